@@ -1,8 +1,8 @@
 // Boundary-transfer form of vort2flux! (src/fluid-operators/curl.jl:133-165):
 // the edge-vector chain e_ℓ = get_bc!(Δ⁻¹Γ_{ℓ+1}) + R e_{ℓ+1} in a rank-k basis
 // of R = get_bc! ∘ Δ⁻¹ ∘ apply_bc! (mg-utils.jl:7-60), and R's setup.  The
-// transforms around it (the multi-level x- and y-passes, the line samples and
-// the y-pass of the edge source) are in dst_kernels.cuh; the definitions in
+// transforms around it (the multi-level x-passes, the line samples) are in
+// dst_kernels.cuh, the y-solves in ysolve.cu; the definitions in
 // ibpm_internal.cuh.
 #include "ibpm_internal.cuh"
 

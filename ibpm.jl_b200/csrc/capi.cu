@@ -36,8 +36,8 @@ struct ibpm_handle {
     double beta[2] = {1.5, -0.5};
     int nb = 0, nf = 0, nbodies = 0;
     std::vector<int> body_start;
-    DstPlan px{}, py{};
-    bool have_px = false, have_py = false;
+    DstPlan px{};
+    bool have_px = false;
     // state
     double* G[2] = {nullptr, nullptr};     // Γ (ping-pong: state / trial)
     double* Nl[2] = {nullptr, nullptr};    // nonlinear term (ping-pong)
@@ -235,7 +235,7 @@ static SpecParams spec(const ibpm_handle* h, int mode, int f32 = 0) {
     SpecParams sp;
     sp.mode = mode;
     sp.f32 = f32;
-    sp.scale = 1.0 / (4.0 * h->g.nx * h->g.ny);  // laplacian.jl:38
+    sp.scale = 1.0 / (2.0 * h->g.nx);  // the x-transforms' factor (ysolve.cu)
     sp.dt = h->dt;
     for (int l = 0; l < 8; ++l) {
         const double hc = h->h * std::ldexp(1.0, l);
@@ -246,7 +246,7 @@ static SpecParams spec(const ibpm_handle* h, int mode, int f32 = 0) {
 }
 
 // One Poisson-type solve x = S((S b) ./ M .* scale) on the slabs of `map`:
-// x-pass (b → tmp), y-pass with the spectral divide (tmp in place), x-pass
+// x-pass (b → tmp), y-solve (tmp in place), x-pass
 // (tmp → out, stored or subtracted).  b may equal tmp; tmp may equal out.
 static int poisson(ibpm_handle* h, const double* b, SlabMap bmap, double* tmp, SlabMap tmap, double* out,
                    SlabMap omap, int nslabs, int mode, int emit, const double* coarse = nullptr,
@@ -259,7 +259,7 @@ static int poisson(ibpm_handle* h, const double* b, SlabMap bmap, double* tmp, S
     a.load = coarse ? XLOAD_BC : XLOAD_PLAIN; a.emit = XEMIT_STORE;
     const double slab_bytes = 16.0 * g.n1 * g.n2 * nslabs;  // read + write every element once
     LAUNCH(K_DSTX, slab_bytes, launch_dst_x(g, h->px, a, h->st));
-    LAUNCH(K_DSTY, slab_bytes, launch_dst_y(g, h->py, h->px, tmp, tmap, nslabs, spec(h, mode), h->st));
+    LAUNCH(K_DSTY, slab_bytes, launch_y_solve(g, tmp, tmap, nslabs, spec(h, mode), h->st));
     XPassArgs c{};
     c.in = tmp; c.out = out; c.in_map = tmap; c.out_map = omap;
     c.nslabs = nslabs; c.line0 = 0; c.line1 = g.n2;
@@ -398,7 +398,7 @@ static int vort2flux(ibpm_handle* h, double* G, double* psi, long long bstride, 
 // coarser ψ (curl.jl:147-162).  Here every level's interior part Δ⁻¹Γ_ℓ is
 // one multi-level solve; the edge vectors follow from its line samples by the
 // chain e_ℓ = get_bc!(Δ⁻¹Γ_{ℓ+1}) + R e_{ℓ+1} (mg−1 small launches); one
-// y-pass builds every level's edge part from e_ℓ, and one x-pass transforms
+// y-solve builds every level's edge part from e_ℓ, and one x-pass transforms
 // the sum of both parts.  The result is the reference's ψ and q up to
 // rounding (both parts are the same linear operators applied in another
 // order).
@@ -493,9 +493,9 @@ static int upload_bt(ibpm_handle* h, const BtLowRank& lr) {
     return IBPM_OK;
 }
 
-// From the y-pass output Y of every level (x-spectral; FP64 or FP32): the line
+// From the y-solve's output Y of every level (x-spectral; FP64 or FP32): the line
 // samples of levels 1 … mg−1, the edge chain down to level 0, and the edge
-// part of levels 0 … nyb−1 by one y-pass, into btY / btY32.
+// part of levels 0 … nyb−1 by one y-solve, into btY / btY32.
 static int bt_edges(ibpm_handle* h, const void* Y, bool f32, int nyb) {
     const Geom& g = h->g;
     const int mg = g.mg, ns = h->gsim;
@@ -515,7 +515,7 @@ static int bt_edges(ibpm_handle* h, const void* Y, bool f32, int nyb) {
     BtSynth bsy{};
     bsy.e = h->btE; bsy.sx = h->px.s; bsy.nx = g.nx;
     LAUNCH(K_DSTY, es * g.n1 * g.n2 * nyb * ns,
-           launch_dst_ybc(g, h->py, h->px, f32 ? (void*)h->btY32 : (void*)h->btY, levmap(g, 0, nyb, bs), nyb * ns,
+           launch_y_solve_edges(g, f32 ? (void*)h->btY32 : (void*)h->btY, levmap(g, 0, nyb, bs), nyb * ns,
                           spec(h, SPEC_DELTA, f32 ? 1 : 0), bsy, h->st));
     return IBPM_OK;
 }
@@ -549,7 +549,7 @@ static int vort2flux_bt(ibpm_handle* h, double* G, double* q, int qnlev, int nfu
     a.nslabs = mg * ns; a.line0 = 0; a.line1 = g.n2; a.load = XLOAD_PLAIN; a.emit = XEMIT_STORE;
     LAUNCH(K_DSTX, 16.0 * slab * mg * ns, launch_dst_x(g, h->px, a, h->st));
     LAUNCH(K_DSTY, 16.0 * slab * mg * ns,
-           launch_dst_y(g, h->py, h->px, h->rhs, all, mg * ns, spec(h, SPEC_DELTA), h->st));
+           launch_y_solve(g, h->rhs, all, mg * ns, spec(h, SPEC_DELTA), h->st));
     int rc = bt_edges(h, h->rhs, false, std::min(nfull, mg - 1));
     if (rc) return rc;
     SlabMap part = levmap(g, 0, nfull, bs);
@@ -585,7 +585,7 @@ static int vort2flux_refined_bt(ibpm_handle* h, double* G, int nsw, double* q, i
         a.nslabs = mg * ns; a.line0 = 0; a.line1 = g.n2; a.load = XLOAD_F32; a.emit = XEMIT_F32;
         LAUNCH(K_DSTX, 8.0 * slab * mg * ns, launch_dst_x(g, h->px, a, h->st));
         LAUNCH(K_DSTY, 8.0 * slab * mg * ns,
-               launch_dst_y(g, h->py, h->px, h->T32, all, mg * ns, spec(h, SPEC_DELTA, 1), h->st));
+               launch_y_solve(g, h->T32, all, mg * ns, spec(h, SPEC_DELTA, 1), h->st));
         int rc = bt_edges(h, h->T32, true, std::min(nfull, mg - 1));
         if (rc) return rc;
         XPassArgs c{};
@@ -665,7 +665,7 @@ static int correction32(ibpm_handle* h, int load, const double* b, const double*
     a.nslabs = ns; a.line0 = 0; a.line1 = g.n2; a.load = load; a.emit = XEMIT_F32;
     LAUNCH(K_DSTX, slab * (8.0 + 8.0 + 4.0), launch_dst_x(g, h->px, a, h->st));
     LAUNCH(K_DSTY, slab * 8.0,
-           launch_dst_y(g, h->py, h->px, h->T32, m, ns, spec(h, load == XLOAD_RES_A ? SPEC_AINV : SPEC_DELTA, 1),
+           launch_y_solve(g, h->T32, m, ns, spec(h, load == XLOAD_RES_A ? SPEC_AINV : SPEC_DELTA, 1),
                         h->st));
     XPassArgs c{};
     c.in = h->T32; c.out = out; c.in_map = m; c.out_map = m;
@@ -883,12 +883,10 @@ static int build_binv(ibpm_handle* h) {
     // B at create is built with the single-level (latency) plan on every
     // launch, so B⁻¹, and every step it feeds, does not depend on the
     // multi-level plan chosen for the steps
-    const int planN[2] = {h->px.planN, h->py.planN};
+    const int planN = h->px.planN;
     h->px.planN = h->px.plan1;
-    h->py.planN = h->py.plan1;
     auto cleanup = [&]() {
-        h->px.planN = planN[0];
-        h->py.planN = planN[1];
+        h->px.planN = planN;
         cudaFree(GB); cudaFree(PB); cudaFree(QB); cudaFree(work); cudaFree(info);
     };
     for (int c0 = 0; c0 < nf && rc == IBPM_OK; c0 += chunk) {
@@ -952,7 +950,6 @@ static void free_handle(ibpm_handle* h) {
     if (h->pin_status) cudaFreeHost(h->pin_status);
     for (cudaEvent_t e : h->prof_ev) cudaEventDestroy(e);
     if (h->have_px) dst_plan_destroy(&h->px);
-    if (h->have_py) dst_plan_destroy(&h->py);
     if (h->st) cudaStreamDestroy(h->st);
     delete h;
 }
@@ -998,10 +995,8 @@ static int create_impl(ibpm_handle* h, const ibpm_problem_desc* d) {
     const char* sup = "32, 64, 128, 192, 200, 256, 384, 400, 512, 768, 1024, 2048";
     if (!dst_supported(g.nx)) return fail(h, IBPM_ERR_UNSUPPORTED, std::string("nx must be one of ") + sup);
     if (!dst_supported(g.ny)) return fail(h, IBPM_ERR_UNSUPPORTED, std::string("ny must be one of ") + sup);
-    if (dst_plan_create(&h->px, g.nx, h->st)) return fail(h, IBPM_ERR_CUDA, "DST plan (x) setup failed");
+    if (dst_plan_create(&h->px, g.nx, h->st)) return fail(h, IBPM_ERR_CUDA, "DST plan setup failed");
     h->have_px = true;
-    if (dst_plan_create(&h->py, g.ny, h->st)) return fail(h, IBPM_ERR_CUDA, "DST plan (y) setup failed");
-    h->have_py = true;
     // base_flux! for inertial motion (timestepping.jl:252-270)
     for (int l = 0; l < g.mg; ++l) {
         const double hc = d->h * std::ldexp(1.0, l);
@@ -1437,10 +1432,8 @@ extern "C" int ibpm_get_binv(ibpm_handle* h, double* Binv) {
 // the default for single-slab launches) or the throughput plan (radix 8).
 // The step graphs are captured again on the next advance.
 static void set_plans(ibpm_handle* h, int single_slab, int multi_slab) {
-    for (DstPlan* p : {&h->px, &h->py}) {
-        p->plan1 = single_slab;
-        p->planN = multi_slab;
-    }
+    h->px.plan1 = single_slab;
+    h->px.planN = multi_slab;
     h->graphs_ready = false;
     for (int p = 0; p < 2; ++p) if (h->gadj[p]) { cudaGraphExecDestroy(h->gadj[p]); h->gadj[p] = nullptr; }
 }
@@ -1644,7 +1637,7 @@ static int solves_T(ibpm_handle* h, const double* qbar, int qnlev, double* Gacc)
         a.in = h->psib; a.out = h->rhs; a.in_map = one; a.out_map = one;
         a.nslabs = 1; a.line0 = 0; a.line1 = g.n2; a.load = XLOAD_PLAIN; a.emit = XEMIT_STORE;
         LAUNCH(K_DSTX, slab, launch_dst_x(g, h->px, a, h->st));
-        LAUNCH(K_DSTY, slab, launch_dst_y(g, h->py, h->px, h->rhs, one, 1, spec(h, SPEC_DELTA), h->st));
+        LAUNCH(K_DSTY, slab, launch_y_solve(g, h->rhs, one, 1, spec(h, SPEC_DELTA), h->st));
         XPassArgs c{};
         c.in = h->rhs; c.out = Gacc; c.in_map = one; c.out_map = m; c.aux = h->Wadj; c.aux_map = m;
         c.nslabs = 1; c.line0 = 0; c.line1 = g.n2; c.load = XLOAD_PLAIN; c.emit = XEMIT_ADD_STORE;
@@ -2163,7 +2156,7 @@ static bool group_shared(const BatchGroup& gr) {
     const ibpm_handle* h0 = gr.mem[0];
     for (auto* h : gr.mem)
         if (h->bt != h0->bt || h->px.plan1 != h0->px.plan1 || h->px.planN != h0->px.planN ||
-            h->py.plan1 != h0->py.plan1 || h->py.planN != h0->py.planN || h->lin || h->moving || h->bodies_moving)
+            h->lin || h->moving || h->bodies_moving)
             return false;
     return true;
 }
@@ -2225,13 +2218,13 @@ static int batch_enqueue_unit(ibpm_batch* b, int u, cudaStream_t st, int p, bool
     cudaStream_t own = h->st;
     h->st = st;
     h->gsim = (int)gr.mem.size(); h->gmem = gr.mem.data();
-    h->px.sims = h->py.sims = h->gsim;
+    h->px.sims = h->gsim;
     h->g_den = gr.den; h->g_cA = gr.cA; h->g_rhs[0] = gr.rhs[0]; h->g_rhs[1] = gr.rhs[1];
     h->g_br = gr.br.data(); h->g_ev = gr.ev.data();
     const int rc = enqueue_step(h, p, cold);
     h->st = own;
     h->gsim = 1; h->gmem = nullptr; h->g_den = nullptr; h->g_cA = nullptr;
-    h->px.sims = h->py.sims = 0;
+    h->px.sims = 0;
     h->g_rhs[0] = h->g_rhs[1] = nullptr; h->g_br = nullptr; h->g_ev = nullptr;
     if (rc) b->err = "group of " + std::to_string(gr.mem.size()) + " members: " + h->err;
     return rc;

@@ -12,11 +12,7 @@ namespace ibpm {
 
 #define IBPM_DST_DECLARE(N)                                                                                   \
     cudaError_t dst_x_##N(const Geom&, const DstPlan&, const XPassArgs&, cudaStream_t);                      \
-    cudaError_t dst_y_##N(const Geom&, const DstPlan&, const DstPlan&, void*, SlabMap, int, const SpecParams&, \
-                          cudaStream_t);                                                                     \
     cudaError_t dst_attr_##N();                                                                              \
-    cudaError_t dst_ybc_##N(const Geom&, const DstPlan&, const DstPlan&, void*, SlabMap, int, const SpecParams&, \
-                            const BtSynth&, cudaStream_t);                                                   \
     cudaError_t dst_lines_##N(const Geom&, const DstPlan&, const void*, SlabMap, int, void*, int, cudaStream_t);
 IBPM_DST_LENGTHS(IBPM_DST_DECLARE)
 #undef IBPM_DST_DECLARE
@@ -156,28 +152,6 @@ cudaError_t dst_init_attributes(int N) {
 cudaError_t launch_dst_x(const Geom& g, const DstPlan& px, const XPassArgs& a, cudaStream_t st) {
     switch (px.N) {
 #define IBPM_CASE(L) case L: return dst_x_##L(g, px, a, st);
-        IBPM_DST_LENGTHS(IBPM_CASE)
-#undef IBPM_CASE
-        default: return cudaErrorInvalidValue;
-    }
-}
-
-cudaError_t launch_dst_y(const Geom& g, const DstPlan& py, const DstPlan& px, void* data, SlabMap map, int nslabs,
-                         const SpecParams& sp, cudaStream_t st) {
-    if (nslabs <= 0) return cudaSuccess;
-    switch (py.N) {
-#define IBPM_CASE(L) case L: return dst_y_##L(g, py, px, data, map, nslabs, sp, st);
-        IBPM_DST_LENGTHS(IBPM_CASE)
-#undef IBPM_CASE
-        default: return cudaErrorInvalidValue;
-    }
-}
-
-cudaError_t launch_dst_ybc(const Geom& g, const DstPlan& py, const DstPlan& px, void* out, SlabMap map, int nslabs,
-                           const SpecParams& sp, const BtSynth& bs, cudaStream_t st) {
-    if (nslabs <= 0) return cudaSuccess;
-    switch (py.N) {
-#define IBPM_CASE(L) case L: return dst_ybc_##L(g, py, px, out, map, nslabs, sp, bs, st);
         IBPM_DST_LENGTHS(IBPM_CASE)
 #undef IBPM_CASE
         default: return cudaErrorInvalidValue;

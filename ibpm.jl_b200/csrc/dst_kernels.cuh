@@ -1,6 +1,7 @@
-// Batched 2-D DST-I (FFTW RODFT00, unnormalised) for the Poisson-type solves of
-// the IBPM step: x = S((S b) ./ M .* scale), S the 2-D DST-I
-// (src/fluid-operators/dst-inversion.jl:39-50, laplacian.jl:24-76).
+// Batched DST-I along x (FFTW RODFT00, unnormalised) for the Poisson-type solves
+// of the IBPM step: x = S((S b) ./ M .* scale), S the 2-D DST-I
+// (src/fluid-operators/dst-inversion.jl:39-50, laplacian.jl:24-76); the
+// y-direction is solved per x-mode (ysolve.cu).
 //
 // A 1-D DST-I of length n = N-1,  Y_k = 2 Σ_m f_m sin(π m k / N)  (f_m = X_{m-1}),
 // is computed for TWO real lines at once (f = a + i b) with one complex FFT of
@@ -610,19 +611,15 @@ __global__ void __launch_bounds__(ct_groups(N, PL) * ct_tp(N, PL), ct_fine(N, PL
 }
 
 // ---------------------------------------------------------------------------
-// y-pass of a Poisson-type solve on a tile of TW = 2G columns (all rows)
-// staged in shared memory, in place: DST-I, spectral divide, DST-I.
+// Layout of a shared-memory tile of TW = 2G columns (all rows) that G groups
+// transform along y, each a column pair.  No kernel stages such a tile any more
+// (the y-direction is a tridiagonal solve in registers, ysolve.cu); the layout
+// helpers stay for the bank-conflict checks built on them.
 // ---------------------------------------------------------------------------
-// Groups (column pairs) per CTA of the y-pass.  FP32 passes take one group
-// (more CTAs for a single slab: the refined step's y-passes are single-slab
-// and latency-bound); FP64 passes keep at least two with the fine plan, so a
-// CTA reads tiles of four 8-byte columns.
 template <int N, class T, int PL>
 __host__ __device__ constexpr int y_groups() {
     return (std::is_same<T, double>::value && ct_fine(N, PL) && ct_groups(N, PL) < 2) ? 2 : ct_groups(N, PL);
 }
-template <int N, class T, int PL>
-__host__ __device__ constexpr int y_threads() { return y_groups<N, T, PL>() * ct_tp(N, PL); }
 template <int N, class T, int PL>
 __host__ __device__ constexpr int y_tile_w() { return 2 * y_groups<N, T, PL>(); }
 __host__ __device__ constexpr int round4(int n) { return ((n + 3) / 4) * 4; }
@@ -661,223 +658,9 @@ template <int N, class T, int PL>
 __host__ __device__ constexpr int y_tile_elems(int n2) {
     return round4(2 * y_groups<N, T, PL>() * y_col_stride<N, T, PL>(n2));
 }
-// Scratch of the edge-source synthesis (SYNTH): per-warp partial sums of the
-// bottom and top rows' sine transforms, then the sums themselves.
-template <int N, class T, int PL>
-__host__ __device__ constexpr int y_synth_slots() {
-    return (y_threads<N, T, PL>() / 32 + 2) * 2 * y_tile_w<N, T, PL>();
-}
-template <int N, class T, int PL, bool SYNTH = false>
-__host__ __device__ constexpr size_t y_smem_bytes(int n2) {
-    return tables_bytes<N, T, PL>() + (size_t)round4(n2) * sizeof(T) +  // spectral table of y
-           (size_t)y_tile_elems<N, T, PL>(n2) * sizeof(T) +
-           (size_t)y_groups<N, T, PL>() * ct_buf(N) * sizeof(cplx_t<T>) +
-           (SYNTH ? (size_t)y_synth_slots<N, T, PL>() * sizeof(double) : 0);
-}
-
-// SYNTH: the input is not read but built, the x-spectrum of apply_bc!(e_ℓ)
-// for the edge vector of the slab's level (BtSynth): with S(i, k) =
-// 2 sin(π i k / nx) the x-pass's sine transform,
-//     X(k, j) = S(1, k) e_L(j) + S(nx−1, k) e_R(j)
-//             + [j = 1] Σ_i S(i, k) e_B(i) + [j = ny−1] Σ_i S(i, k) e_T(i),
-// and the result goes to `out` (same slab map) instead of back into `data`.
-template <int N, class T, int PL, bool SYNTH = false>
-// (3 resident 256-thread CTAs per SM keep the FP64 pass at 80 registers without
-// spills: the five-slab trial solve's y-pass then needs 1.4 waves instead of 2.2)
-__global__ void __launch_bounds__(y_threads<N, T, PL>(),
-                                  N > 512 ? 1 : (!ct_fine(N, PL) ? IBPM_WIDE_MIN_BLOCKS
-                                                                 : (y_threads<N, T, PL>() <= 128 ? 5 : 3)))
-    dst_y_kernel(T* data, SlabMap map, Geom g, DstPlan p, const T* __restrict__ cx, SpecParams sp,
-                 T* out = nullptr, BtSynth bs = BtSynth{}) {
-    using V = cplx_t<T>;
-    constexpr int TP = ct_tp(N, PL);
-    constexpr int G = y_groups<N, T, PL>();
-    constexpr int TW = y_tile_w<N, T, PL>();
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int P = g.P, n1 = g.n1, n2 = g.n2;
-    const Tabs<T> tb = tabs_of<T>(p, PL);
-    V* tw = reinterpret_cast<V*>(smem_raw);
-    T* sn = reinterpret_cast<T*>(tw + ct_tw_count(N, PL));
-    T* cyv = reinterpret_cast<T*>(smem_raw + tables_bytes<N, T, PL>());
-    T* tile = cyv + round4(n2);
-    const int tile_d = y_tile_elems<N, T, PL>(n2);
-    constexpr int CS = y_col_stride<N, T, PL>(N - 1);   // n2 = N − 1 in the y-pass
-    auto off = [](int j) -> int { return y_off<N, T, PL>(j); };   // row j within a column
-    auto at = [&](int j, int c) -> int { return c * CS + off(j); };
-    const int gid = threadIdx.x / TP, tid = threadIdx.x % TP;
-    V* buf = reinterpret_cast<V*>(tile + tile_d) + gid * ct_buf(N);
-    const int i0 = blockIdx.x * TW;
-    T* base = data + map.off(blockIdx.y);
-    const int lev = map.level(blockIdx.y);
-
-    stage_tables<N, T, PL>(tw, sn, tb);  // constant tables: before the dependency wait
-    for (int j = threadIdx.x; j < n2; j += blockDim.x) cp_async<sizeof(T)>(cyv + j, tb.c + j);
-    pdl_wait();
-    pdl_trigger();
-    if constexpr (SYNTH) {
-        // the edge vectors and the sums over them are FP64 (they couple the
-        // levels); the tile takes the x-spectrum rounded to T
-        const int ep = ((2 * n1 + 2 * n2) + 3) & ~3;
-        const double* e = static_cast<const double*>(bs.e) + ((long long)map.batch(blockIdx.y) * g.mg + lev) * ep;
-        const double* sxt = static_cast<const double*>(bs.sx);
-        const int nx = bs.nx, nx2 = 2 * bs.nx;
-        auto sinpix = [&](int t) -> double {  // sin(π t / nx), 0 ≤ t < 2 nx
-            return t < nx ? __ldg(&sxt[t]) : -__ldg(&sxt[t - nx]);
-        };
-        double* red = reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(tile + tile_d) +
-                                                (size_t)G * ct_buf(N) * sizeof(V));
-        // bottom and top rows: Σ_i S(i, k) e(i) for the CTA's columns k, the
-        // sine argument (i + 1) k mod 2nx advanced by a fixed step per thread
-        double accB[TW], accT[TW];
-        int tk[TW], dk[TW];
-#pragma unroll
-        for (int c = 0; c < TW; ++c) {
-            accB[c] = accT[c] = 0.0;
-            const int k = i0 + c + 1;
-            tk[c] = (int)(((long long)(threadIdx.x + 1) * k) % nx2);
-            dk[c] = (int)(((long long)blockDim.x * k) % nx2);
-        }
-#pragma unroll 4
-        for (int i = threadIdx.x; i < n1; i += blockDim.x) {
-            const double eb = __ldg(&e[i]), et = __ldg(&e[n1 + i]);
-#pragma unroll
-            for (int c = 0; c < TW; ++c) {
-                const double sv = 2.0 * sinpix(tk[c]);
-                accB[c] += sv * eb;
-                accT[c] += sv * et;
-                tk[c] += dk[c];
-                if (tk[c] >= nx2) tk[c] -= nx2;
-            }
-        }
-        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-        for (int c = 0; c < TW; ++c) {
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                accB[c] += __shfl_xor_sync(0xffffffffu, accB[c], off);
-                accT[c] += __shfl_xor_sync(0xffffffffu, accT[c], off);
-            }
-            if (lane == 0) {
-                red[w * 2 * TW + c] = accB[c];
-                red[w * 2 * TW + TW + c] = accT[c];
-            }
-        }
-        __syncthreads();
-        if (threadIdx.x < 2 * TW) {
-            double acc = 0.0;
-            for (int u = 0; u < nw; ++u) acc += red[u * 2 * TW + threadIdx.x];
-            red[nw * 2 * TW + threadIdx.x] = acc;
-        } else if (threadIdx.x < 4 * TW) {
-            // S(1, k) and S(nx − 1, k) of the column c
-            const int c = (threadIdx.x - 2 * TW) >> 1;
-            const long long k = i0 + c + 1;
-            const int t = (int)(((threadIdx.x & 1) ? k * (nx - 1) : k) % nx2);
-            red[(nw + 1) * 2 * TW + (threadIdx.x - 2 * TW)] = 2.0 * sinpix(t);
-        }
-        __syncthreads();
-        const double* bh = red + nw * 2 * TW;         // [0, TW): bottom, [TW, 2TW): top
-        const double* sLR = red + (nw + 1) * 2 * TW;  // [2c]: S(1, k_c), [2c + 1]: S(nx−1, k_c)
-        const double* eL = e + 2 * n1;
-        const double* eR = eL + n2;
-        // (the loads of eight steps in flight: the loop is a chain of L2 reads otherwise)
-#pragma unroll 8
-        for (int idx = threadIdx.x; idx < n2 * TW; idx += blockDim.x) {
-            const int j = idx / TW, c = idx - j * TW;
-            const int i = i0 + c;
-            double v = 0.0;
-            if (i < n1) {
-                v = sLR[2 * c] * __ldg(&eL[j]) + sLR[2 * c + 1] * __ldg(&eR[j]);
-                if (j == 0) v += bh[c];
-                if (j == n2 - 1) v += bh[TW + c];
-            }
-            tile[at(j, c)] = (T)v;
-        }
-        __syncthreads();
-    } else {
-        for (int idx = threadIdx.x; idx < n2 * TW; idx += blockDim.x) {
-            const int j = idx / TW, c = idx - j * TW;
-            const int i = i0 + c;
-            if (i < n1) cp_async<sizeof(T)>(tile + at(j, c), base + (long long)j * P + i);
-            else tile[at(j, c)] = T(0);
-        }
-        cp_async_wait();
-        __syncthreads();
-    }
-
-    const int ca = 2 * gid;
-    const int ia = i0 + ca;
-    if (ia < n1) {
-        const bool hasb = ia + 1 < n1;
-        T* const colA = tile + ca * CS;   // the group's two columns
-        T* const colB = colA + CS;
-        auto load = [&](int m) -> V { return V{colA[off(m)], colB[off(m)]}; };
-        auto emit = [&](int o, V v) {
-            colA[off(o)] = v.x;
-            colB[off(o)] = v.y;
-        };
-        auto divide = [&]() {
-            if constexpr (std::is_same<T, double>::value) {
-                // w ./= M ; w .*= scale  with Λ = -2 (cos(π i/nx) + cos(π j/ny) - 2)
-                // (laplacian.jl:17-41, 61-71)
-                const double cxa = __ldg(&cx[ia]);
-                const double cxb = hasb ? __ldg(&cx[ia + 1]) : 0.0;
-                const double* md = sp.mden ? sp.mden + (long long)map.batch(blockIdx.y) * 9 : nullptr;
-                const double den = md ? md[lev] : sp.den[lev];
-                const double dt = md ? md[8] : sp.dt;
-                for (int o = tid; o < n2; o += TP) {
-                    const double c2 = cyv[o];
-                    const double la = -2.0 * ((cxa + c2) - 2.0);
-                    const double lb = -2.0 * ((cxb + c2) - 2.0);
-                    double Ma, Mb;
-                    if (sp.mode == SPEC_DELTA) {
-                        Ma = la;
-                        Mb = lb;
-                    } else {
-                        Ma = 1.0 + la * dt / den;
-                        Mb = 1.0 + lb * dt / den;
-                    }
-                    const int oo = off(o);
-                    colA[oo] = (colA[oo] * nr_rcp(Ma)) * sp.scale;
-                    colB[oo] = hasb ? (colB[oo] * nr_rcp(Mb)) * sp.scale : 0.0;
-                }
-            } else {
-                // the same divisor from Λ = a_x(i) + a_y(j), a(k) = 4 sin²(πk/(2n)):
-                // no cancellation for the smallest eigenvalues in FP32
-                const float axa = __ldg(&cx[ia]);
-                const float axb = hasb ? __ldg(&cx[ia + 1]) : 0.0f;
-                const double* md = sp.mden ? sp.mden + (long long)map.batch(blockIdx.y) * 9 : nullptr;
-                const float kf = (sp.mode == SPEC_DELTA) ? 0.0f
-                                 : md ? (float)(md[8] / md[lev]) : (float)(sp.dt / sp.den[lev]);
-                const float sc = (float)sp.scale;
-                for (int o = tid; o < n2; o += TP) {
-                    const float la = axa + cyv[o];
-                    const float lb = axb + cyv[o];
-                    const float Ma = (sp.mode == SPEC_DELTA) ? la : fmaf(la, kf, 1.0f);
-                    const float Mb = (sp.mode == SPEC_DELTA) ? lb : fmaf(lb, kf, 1.0f);
-                    const int oo = off(o);
-                    colA[oo] = colA[oo] * (__frcp_rn(Ma) * sc);
-                    colB[oo] = hasb ? colB[oo] * (__frcp_rn(Mb) * sc) : 0.0f;
-                }
-            }
-        };
-        dst_pair<N, TP, G, T, PL>(buf, tw, sn, tid, gid, load, emit);
-        gsync<TP, G>(gid);
-        divide();
-        gsync<TP, G>(gid);
-        dst_pair<N, TP, G, T, PL>(buf, tw, sn, tid, gid, load, emit);
-    }
-    __syncthreads();
-    T* dst = SYNTH ? out + map.off(blockIdx.y) : base;
-    for (int idx = threadIdx.x; idx < n2 * TW; idx += blockDim.x) {
-        const int j = idx / TW, c = idx - j * TW;
-        const int i = i0 + c;
-        if (i < n1) dst[(long long)j * P + i] = tile[at(j, c)];
-    }
-}
-
 // ---------------------------------------------------------------------------
 // Line samples of a boundary-transfer vort2flux! (ibpm_internal.cuh, BtSynth)
-// from the y-pass output Y (x-spectral, y-physical) of the levels of `map`:
+// from the y-solve's output Y (x-spectral, y-physical) of the levels of `map`:
 // block 0 of a slab transforms the rows at ny/4 and at 3ny/4 back along x (one
 // line pair) and keeps x = nx/4 … 3nx/4; the other blocks form the columns at
 // nx/4 and 3nx/4, ψ(i0, j) = Σ_k S(i0, k) Y(k, j), one warp per row j.  There
@@ -1005,48 +788,6 @@ cudaError_t launch_x_t(const Geom& g, const DstPlan& px, const XPassArgs& a, cud
 }
 
 template <int N, class T, int PL>
-cudaError_t launch_y_n(const Geom& g, const DstPlan& py, const DstPlan& px, void* data, SlabMap map, int nslabs,
-                       const SpecParams& sp, cudaStream_t st) {
-    constexpr int TW = y_tile_w<N, T, PL>();
-    if (g.n2 != N - 1) return cudaErrorInvalidValue;   // the tile's column stride is fixed by N
-    const size_t smem = y_smem_bytes<N, T, PL>(g.n2);
-    if (smem > 227 * 1024) return cudaErrorInvalidConfiguration;
-    dim3 grid((g.n1 + TW - 1) / TW, nslabs);
-    const int threads = y_threads<N, T, PL>();
-    return launch_k(dst_y_kernel<N, T, PL>, grid, dim3(threads), smem, st, static_cast<T*>(data), map, g, py,
-                    static_cast<const T*>(tabs_of<T>(px).c), sp, static_cast<T*>(nullptr), BtSynth{});
-}
-
-template <int N>
-cudaError_t launch_y_t(const Geom& g, const DstPlan& py, const DstPlan& px, void* data, SlabMap map, int nslabs,
-                       const SpecParams& sp, cudaStream_t st) {
-    IBPM_PLAN_SWITCH(N, launch_plan(N, py, nslabs),
-                     return sp.f32 ? launch_y_n<N, float, PLN>(g, py, px, data, map, nslabs, sp, st)
-                                   : launch_y_n<N, double, PLN>(g, py, px, data, map, nslabs, sp, st))
-}
-
-template <int N, class T, int PL>
-cudaError_t launch_ybc_n(const Geom& g, const DstPlan& py, const DstPlan& px, void* out, SlabMap map, int nslabs,
-                         const SpecParams& sp, const BtSynth& bs, cudaStream_t st) {
-    constexpr int TW = y_tile_w<N, T, PL>();
-    if (g.n2 != N - 1) return cudaErrorInvalidValue;   // the tile's column stride is fixed by N
-    const size_t smem = y_smem_bytes<N, T, PL, true>(g.n2);
-    if (smem > 227 * 1024) return cudaErrorInvalidConfiguration;
-    dim3 grid((g.n1 + TW - 1) / TW, nslabs);
-    return launch_k(dst_y_kernel<N, T, PL, true>, grid, dim3(y_threads<N, T, PL>()), smem, st,
-                    static_cast<T*>(nullptr), map, g, py, static_cast<const T*>(tabs_of<T>(px).c), sp,
-                    static_cast<T*>(out), bs);
-}
-
-template <int N>
-cudaError_t launch_ybc_t(const Geom& g, const DstPlan& py, const DstPlan& px, void* out, SlabMap map, int nslabs,
-                         const SpecParams& sp, const BtSynth& bs, cudaStream_t st) {
-    IBPM_PLAN_SWITCH(N, launch_plan(N, py, nslabs),
-                     return sp.f32 ? launch_ybc_n<N, float, PLN>(g, py, px, out, map, nslabs, sp, bs, st)
-                                   : launch_ybc_n<N, double, PLN>(g, py, px, out, map, nslabs, sp, bs, st))
-}
-
-template <int N, class T, int PL>
 cudaError_t launch_lines_n(const Geom& g, const DstPlan& px, const void* Y, SlabMap map, int nslabs, void* smp,
                            cudaStream_t st) {
     constexpr int TP = ct_tp(N, PL);
@@ -1078,12 +819,8 @@ cudaError_t attr_plan() {
     if ((e = smem_attrs(dst_x_kernel<N, L, E, PL>))) return e;
     IBPM_X_COMBOS(IBPM_X_ATTR)
 #undef IBPM_X_ATTR
-    if ((e = smem_attrs(dst_y_kernel<N, double, PL>))) return e;
-    if ((e = smem_attrs(dst_y_kernel<N, double, PL, true>))) return e;
-    if ((e = smem_attrs(dst_y_kernel<N, float, PL, true>))) return e;
     if ((e = smem_attrs(dst_lines_kernel<N, double, PL>))) return e;
-    if ((e = smem_attrs(dst_lines_kernel<N, float, PL>))) return e;
-    return smem_attrs(dst_y_kernel<N, float, PL>);
+    return smem_attrs(dst_lines_kernel<N, float, PL>);
 }
 
 template <int N>
@@ -1101,15 +838,7 @@ cudaError_t attr_t() {
     cudaError_t dst_x_##N(const Geom& g, const DstPlan& px, const XPassArgs& a, cudaStream_t st) {         \
         return dstk::launch_x_t<N>(g, px, a, st);                                                          \
     }                                                                                                      \
-    cudaError_t dst_y_##N(const Geom& g, const DstPlan& py, const DstPlan& px, void* d, SlabMap m, int n,   \
-                          const SpecParams& sp, cudaStream_t st) {                                         \
-        return dstk::launch_y_t<N>(g, py, px, d, m, n, sp, st);                                            \
-    }                                                                                                      \
     cudaError_t dst_attr_##N() { return dstk::attr_t<N>(); }                                               \
-    cudaError_t dst_ybc_##N(const Geom& g, const DstPlan& py, const DstPlan& px, void* o, SlabMap m, int n,  \
-                            const SpecParams& sp, const BtSynth& bs, cudaStream_t st) {                     \
-        return dstk::launch_ybc_t<N>(g, py, px, o, m, n, sp, bs, st);                                      \
-    }                                                                                                      \
     cudaError_t dst_lines_##N(const Geom& g, const DstPlan& px, const void* Y, SlabMap m, int n, void* smp, \
                               int f32, cudaStream_t st) {                                                  \
         return dstk::launch_lines_t<N>(g, px, Y, m, n, smp, f32, st);                                      \

@@ -163,7 +163,7 @@ cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t sme
 // Host-side launchers (defined in the .cu files).
 // ---------------------------------------------------------------------------
 struct DstPlan {
-    int N;               // transform length nx (x-pass) or ny (y-pass) = n + 1
+    int N;               // transform length nx = n1 + 1
     double2* W;          // device: per-stage FFT twiddles (stage-contiguous, ≤ N entries)
     double* s;           // device: sin(π m/N), m < N
     double* c;           // device: cos(π (k+1)/N), k < N-1 (Laplacian eigenvalues)
@@ -203,14 +203,15 @@ DstPlan dst_plan_at(double* base, int N);
 void set_global_error(const char* msg);
 void dst_plan_destroy(DstPlan* p);
 
-// Spectral divisor applied between the two y-transforms of a Poisson solve:
-//   DELTA: w ← (w / Λ) · scale                       (Δ⁻¹, laplacian.jl:24-41)
-//   AINV:  w ← (w / (1 + Λ·dt / den[lev])) · scale    (A⁻¹, laplacian.jl:61-71)
+// Operator of a y-solve (ysolve.cu) on x-spectral data, with the scale of the
+// two x-transforms around it:
+//   DELTA: Δ⁻¹ (laplacian.jl:24-41)
+//   AINV:  A⁻¹ = (I + c Δ)⁻¹, c = dt / den[lev] (laplacian.jl:61-71)
 enum SpecMode { SPEC_DELTA = 0, SPEC_AINV = 1 };
 struct SpecParams {
     int mode;
-    int f32;             // data and transforms in FP32 (the refinement correction)
-    double scale;        // 1 / (4 nx ny)
+    int f32;             // data in FP32 (the refinement correction); the solve itself is FP64
+    double scale;        // 1 / (2 nx)
     double dt;
     double den[8];       // 2 Re hc² per level
     // a launch over the slabs of several simulations of one grid (batch
@@ -259,10 +260,9 @@ cudaError_t launch_dst_x(const Geom& g, const DstPlan& px, const XPassArgs& a, c
 
 
 
-// y-direction pass of a Poisson-type solve, in place on every slab selected by
-// `map`: DST-I, spectral divide (SpecParams), DST-I.
-cudaError_t launch_dst_y(const Geom& g, const DstPlan& py, const DstPlan& px_cos, void* data, SlabMap map,
-                         int nslabs, const SpecParams& sp, cudaStream_t st);
+// y-direction of a Poisson-type solve (ysolve.cu), in place on every x-spectral
+// slab selected by `map`: per x-mode the tridiagonal solve along y.
+cudaError_t launch_y_solve(const Geom& g, void* data, SlabMap map, int nslabs, const SpecParams& sp, cudaStream_t st);
 
 // ---------------------------------------------------------------------------
 // Boundary-transfer form of vort2flux! (bt.cu).  Δ⁻¹ is linear, so each
@@ -275,10 +275,10 @@ cudaError_t launch_dst_y(const Geom& g, const DstPlan& py, const DstPlan& px_cos
 // apply_bc! adds: bottom i = 1…nx−1, top, left j = 1…ny−1, right.
 // The x-spectrum of apply_bc!(e) is known in closed form (one sine transform
 // of the bottom and top rows, two sines for the left and right columns), so
-// the edge part is one y-pass from e and the last x-pass adds both parts.
+// the edge part is one y-solve from e and the last x-pass adds both parts.
 // Line samples of a level (what get_bc! reads from it): the row at ny/4 and
 // at 3ny/4 (x = nx/4 … 3nx/4, nx/2+1 values each), then the column at nx/4 and
-// at 3nx/4 (y = ny/4 … 3ny/4), each taken from the y-pass output (x-spectral).
+// at 3nx/4 (y = ny/4 … 3ny/4), each taken from the y-solve's output (x-spectral).
 // ---------------------------------------------------------------------------
 inline int bt_edge_len(const Geom& g) { return 2 * g.n1 + 2 * g.n2; }
 inline int bt_edge_pitch(const Geom& g) { return (bt_edge_len(g) + 3) & ~3; }  // R row pitch
@@ -288,8 +288,9 @@ struct BtSynth {
     const double* sx;     // sin(π t/nx), t < nx, of the x-length (FP64)
     int nx;
 };
-cudaError_t launch_dst_ybc(const Geom& g, const DstPlan& py, const DstPlan& px, void* out, SlabMap map, int nslabs,
-                           const SpecParams& sp, const BtSynth& bs, cudaStream_t st);
+// The y-solve of the edge vectors' x-spectrum into the slabs of `out`.
+cudaError_t launch_y_solve_edges(const Geom& g, void* out, SlabMap map, int nslabs, const SpecParams& sp,
+                                 const BtSynth& bs, cudaStream_t st);
 // The line samples (FP64) of the levels of `map` from Y (FP32 when f32).
 cudaError_t launch_dst_lines(const Geom& g, const DstPlan& px, const void* Y, SlabMap map, int nslabs,
                              void* samples, int f32, cudaStream_t st);

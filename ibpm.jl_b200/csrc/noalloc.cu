@@ -90,9 +90,8 @@ extern "C" int ibpm_lap_inv_noalloc(int32_t nx, int32_t ny, const double* rhs, d
         ds.ready = true;
     }
     double* tx = ds.tables + table_offset(length_index(nx));
-    double* ty = ds.tables + table_offset(length_index(ny));
     const Geom g = make_geom(nx, ny, 1);
-    const DstPlan px = dst_plan_at(tx, nx), py = dst_plan_at(ty, ny);
+    const DstPlan px = dst_plan_at(tx, nx);
     // Every slab element that the transforms read (columns < nx-1) is written
     // by this copy, so nothing left by an earlier call is read.
     const size_t row = sizeof(double) * g.n1;
@@ -105,9 +104,9 @@ extern "C" int ibpm_lap_inv_noalloc(int32_t nx, int32_t ny, const double* rhs, d
     a.nslabs = 1; a.line0 = 0; a.line1 = g.n2; a.load = XLOAD_PLAIN; a.emit = XEMIT_STORE;
     SpecParams sp{};
     sp.mode = SPEC_DELTA;
-    sp.scale = 1.0 / (4.0 * nx * ny);  // get_lap_inv, laplacian.jl:38
+    sp.scale = 1.0 / (2.0 * nx);  // the x-transforms' factor (ysolve.cu)
     if ((e = launch_dst_x(g, px, a, st)) != cudaSuccess ||
-        (e = launch_dst_y(g, py, px, ds.slab, m, 1, sp, st)) != cudaSuccess ||
+        (e = launch_y_solve(g, ds.slab, m, 1, sp, st)) != cudaSuccess ||
         (e = launch_dst_x(g, px, a, st)) != cudaSuccess)
         return noalloc_fail(IBPM_ERR_CUDA, std::string("solve: ") + cudaGetErrorString(e));
     e = cudaMemcpy2DAsync(x, row, ds.slab, sizeof(double) * g.P, row, g.n2, cudaMemcpyDeviceToDevice, st);
