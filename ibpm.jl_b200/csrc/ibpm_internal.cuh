@@ -97,6 +97,30 @@ struct CoarseBC {
     }
 };
 
+// Fluxes q = C ψ of one level at 1-based (I, J) with the edge streamfunction
+// ψbc = get_bc!(ψ[lev+1]) (curl.jl:81-116), the bottom row of x-fluxes reading
+// ψbc[(B-1)+i] (curl.jl:92), i.e. edge vertex i-2, where the top row reads i-1.
+struct CurlAt {
+    const double* psi;
+    int P, nx, ny;
+    CoarseBC eb;
+    __device__ __forceinline__ double ps(int I, int J) const { return psi[(long long)(J - 1) * P + (I - 1)]; }
+    __device__ __forceinline__ double x(int I, int J) const {
+        if (I == 1) return eb.left(J) - eb.left(J - 1);
+        if (I == nx + 1) return eb.right(J) - eb.right(J - 1);
+        if (J == 1) return ps(I - 1, 1) - eb.bot(I - 2);
+        if (J == ny) return eb.top(I - 1) - ps(I - 1, ny - 1);
+        return ps(I - 1, J) - ps(I - 1, J - 1);
+    }
+    __device__ __forceinline__ double y(int I, int J) const {
+        if (J == 1) return eb.bot(I - 1) - eb.bot(I);
+        if (J == ny + 1) return eb.top(I - 1) - eb.top(I);
+        if (I == 1) return eb.left(J - 1) - ps(1, J - 1);
+        if (I == nx) return ps(nx - 1, J - 1) - eb.right(J - 1);
+        return ps(I - 1, J - 1) - ps(I, J - 1);
+    }
+};
+
 // ---------------------------------------------------------------------------
 // Programmatic dependent launch: every kernel of the step is launched with
 // cudaLaunchAttributeProgrammaticStreamSerialization, so it can be scheduled

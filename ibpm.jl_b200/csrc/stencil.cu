@@ -17,6 +17,14 @@ namespace ibpm {
 // through two DSTs with the eigenvalues 1 − Λ c (laplacian.jl:73-76), whose
 // eigenvectors are exactly the DST-I basis.
 // ---------------------------------------------------------------------------
+// In N = C' fq the product at the point's own vertex enters both x-faces (and
+// both y-faces) with opposite signs, so only the four neighbours are left:
+//   4 hc² N = Qy(i+1, j) Γ(i, j−1) − Qy(i+1, j+2) Γ(i, j+1)
+//           + Qx(i, j+1) Γ(i−1, j) − Qx(i+2, j+1) Γ(i+1, j),
+// 13 loads per point with the stencil's, where forming the four products of fq
+// read about 30 values and tested for the edges at each (five levels of 511²
+// 31 -> 22 µs, of 1023² 108 -> 73 µs, timed by events in the step; the bytes of
+// the latter, 252 MB, take 39 µs).  Bound by L1 and L2 requests.
 // LIN: the linearised problem's term (nonlinear.jl:45-65, 144-163),
 //   N = C'(DP(Q, ΓB) + DP(QB, Γ)) / (4 hc²),
 // Q the face sums of q without base flux, QB those of the base state with its
@@ -26,7 +34,8 @@ namespace ibpm {
 // GRP: the simulations of a batch group, blockIdx.z = simulation · mg + level,
 // each with its own arguments in ga[simulation] (its fields, coefficients).
 template <bool LIN, bool MOV, bool GRP = false>
-__global__ void __launch_bounds__(256) trial_rhs_kernel(RhsArgs a0, const RhsArgs* __restrict__ ga, Geom g) {
+__global__ void __launch_bounds__(256) trial_rhs_kernel(const __grid_constant__ RhsArgs a0,
+                                                        const RhsArgs* __restrict__ ga, Geom g) {
     pdl_wait();
     pdl_trigger();
     const RhsArgs& a = GRP ? ga[blockIdx.z / g.mg] : a0;
@@ -37,96 +46,75 @@ __global__ void __launch_bounds__(256) trial_rhs_kernel(RhsArgs a0, const RhsArg
     if (i0 >= n1 || j0 >= n2) return;
     const double* G = a.G + a.Gmap.off(lev);
     const double* q = a.q + (long long)lev * g.nq;
-    const double* qy = q + g.nu;
-    const double q0x = a.q0x[lev], q0y = a.q0y[lev];
-    // moving grid: the base flux varies along y on x-faces and along x on y-faces
-    const double* mrow = MOV ? moving_row(a.mv) : nullptr;
-    const double hc = MOV ? ldexp(a.mv.h, lev) : 0.0;
+    const int o = j0 * P + i0;                           // a level is below 2^31 values
+    const int ox = j0 * (nx + 1) + i0;                   // 0-based flux (i0, j0) of the x-faces
+    const int oy = j0 * nx + i0;                         // … of the y-faces
 
-    CoarseBC cb;
-    cb.rc = (lev < a.mg - 1) ? a.G + a.Gmap.off(lev + 1) : nullptr;
-    cb.P = P; cb.nx = nx; cb.ny = ny;
-
-    // Γ extended by the (0.25-scaled) edge values, vertex indices 0 … nx, 0 … ny.
-    auto Ge = [&](int vi, int vj) -> double {
-        if (vj == 0) return 0.25 * cb.bot(vi);
-        if (vj == ny) return 0.25 * cb.top(vi);
-        if (vi == 0) return 0.25 * cb.left(vj);
-        if (vi == nx) return 0.25 * cb.right(vj);
-        return G[(long long)(vj - 1) * P + (vi - 1)];
+    // Γ at the point and its four neighbours: the edge values ¼ get_bc! beyond
+    // the level's edges for the products (gs …), zero for the viscous term (zs …)
+    const double gc = G[o];
+    double gw, ge, gs, gn, zw, ze, zs, zn, rbc = 0.0;
+    if (i0 > 0 && i0 < n1 - 1 && j0 > 0 && j0 < n2 - 1) {
+        zw = gw = G[o - 1];
+        ze = ge = G[o + 1];
+        zs = gs = G[o - P];
+        zn = gn = G[o + P];
+    } else {
+        CoarseBC cb;
+        cb.rc = (lev < a.mg - 1) ? a.G + a.Gmap.off(lev + 1) : nullptr;
+        cb.P = P; cb.nx = nx; cb.ny = ny;
+        // apply_bc!(rhsbc = 0, bc, fac) (mg-utils.jl:43-60), in the order bottom, top, left, right
+        const double fac = a.fac_bc[lev];
+        zs = zn = zw = ze = 0.0;
+        if (j0 == 0) { const double b = cb.bot(i0 + 1); gs = 0.25 * b; rbc += fac * b; }
+        else zs = gs = G[o - P];
+        if (j0 == n2 - 1) { const double b = cb.top(i0 + 1); gn = 0.25 * b; rbc += fac * b; }
+        else zn = gn = G[o + P];
+        if (i0 == 0) { const double b = cb.left(j0 + 1); gw = 0.25 * b; rbc += fac * b; }
+        else zw = gw = G[o - 1];
+        if (i0 == n1 - 1) { const double b = cb.right(j0 + 1); ge = 0.25 * b; rbc += fac * b; }
+        else ze = ge = G[o + 1];
+    }
+    // face sums of avg_flux (nonlinear.jl:17-38) at the four faces, without
+    // base flux: Qx of rows j, j+1 at x-faces I = i, i+2; Qy of columns i, i+1
+    // at y-faces J = j, j+2 (1-based; 0-based offsets below)
+    struct Faces { double w, e, s, n; };
+    auto faces = [&](const double* f) -> Faces {
+        const double* fy = f + g.nu;
+        return {f[ox + nx + 1] + f[ox], f[ox + 2 + nx + 1] + f[ox + 2], fy[oy + 1] + fy[oy],
+                fy[oy + 2 * nx + 1] + fy[oy + 2 * nx]};
     };
-    auto qxJ = [&](int I, int J) -> double { return q[(I - 1) + (long long)(J - 1) * (nx + 1)]; };
-    auto qyJ = [&](int I, int J) -> double { return qy[(I - 1) + (long long)(J - 1) * nx]; };
-    // avg_flux (nonlinear.jl:17-38)
-    auto q0xJ = [&](int J) -> double {
-        if constexpr (MOV) return moving_q0x(a.mv, mrow, J, ny, hc);
-        else return q0x;
-    };
-    auto q0yI = [&](int I) -> double {
-        if constexpr (MOV) return moving_q0y(a.mv, mrow, I, nx, hc);
-        else return q0y;
-    };
-    auto QxJ = [&](int I, int J) -> double { return ((qxJ(I, J) + q0xJ(J)) + qxJ(I, J - 1)) + q0xJ(J - 1); };
-    auto QyJ = [&](int I, int J) -> double { return ((qyJ(I, J) + q0yI(I)) + qyJ(I - 1, J)) + q0yI(I - 1); };
-    // direct_product_loops! (nonlinear.jl:73-114)
-    auto fqxJ = [&](int I, int J) -> double { return QyJ(I, J + 1) * Ge(I - 1, J) + QyJ(I, J) * Ge(I - 1, J - 1); };
-    auto fqyJ = [&](int I, int J) -> double {
-        return -1.0 * (QxJ(I + 1, J) * Ge(I, J - 1) + QxJ(I, J) * Ge(I - 1, J - 1));
-    };
-    const int i = i0 + 1, j = j0 + 1;  // Julia Γ index
+    Faces Q = faces(q);
     double N;
     if constexpr (!LIN) {
-        // C' fq (rot!, curl.jl:22-34) scaled by 1/(4 hc²)
-        N = ((fqxJ(i + 1, j) - fqxJ(i + 1, j + 1)) + (fqyJ(i + 1, j + 1) - fqyJ(i, j + 1))) * a.nl_scale[lev];
+        if constexpr (MOV) {
+            // the base flux varies along y on x-faces and along x on y-faces
+            const double* mrow = moving_row(a.mv);
+            const double hc = ldexp(a.mv.h, lev);
+            const double bx = moving_q0x(a.mv, mrow, j0 + 2, ny, hc) + moving_q0x(a.mv, mrow, j0 + 1, ny, hc);
+            const double by = moving_q0y(a.mv, mrow, i0 + 2, nx, hc) + moving_q0y(a.mv, mrow, i0 + 1, nx, hc);
+            Q.w += bx; Q.e += bx; Q.s += by; Q.n += by;
+        } else {
+            const double bx = 2.0 * a.q0x[lev], by = 2.0 * a.q0y[lev];
+            Q.w += bx; Q.e += bx; Q.s += by; Q.n += by;
+        }
+        N = ((Q.s * gs - Q.n * gn) + (Q.w * gw - Q.e * ge)) * a.nl_scale[lev];
     } else {
-        const double* GB = a.GB + a.Gmap.off(lev);
-        const double* qB = a.qB + (long long)lev * g.nq;
-        const double* qBy = qB + g.nu;
-        const double q0Bx = a.q0Bx[lev], q0By = a.q0By[lev];
-        auto GeB = [&](int vi, int vj) -> double {   // base Γ, this state's edge values
-            if (vj == 0 || vj == ny || vi == 0 || vi == nx) return Ge(vi, vj);
-            return GB[(long long)(vj - 1) * P + (vi - 1)];
-        };
-        auto QxL = [&](int I, int J) -> double { return qxJ(I, J) + qxJ(I, J - 1); };
-        auto QyL = [&](int I, int J) -> double { return qyJ(I, J) + qyJ(I - 1, J); };
-        auto QBx = [&](int I, int J) -> double {
-            return ((qB[(I - 1) + (long long)(J - 1) * (nx + 1)] + q0Bx) + qB[(I - 1) + (long long)(J - 2) * (nx + 1)]) + q0Bx;
-        };
-        auto QBy = [&](int I, int J) -> double {
-            return ((qBy[(I - 1) + (long long)(J - 1) * nx] + q0By) + qBy[(I - 2) + (long long)(J - 1) * nx]) + q0By;
-        };
-        auto fx = [&](int I, int J) -> double {
-            return (QyL(I, J + 1) * GeB(I - 1, J) + QyL(I, J) * GeB(I - 1, J - 1)) +
-                   (QBy(I, J + 1) * Ge(I - 1, J) + QBy(I, J) * Ge(I - 1, J - 1));
-        };
-        auto fy = [&](int I, int J) -> double {
-            return -1.0 * (QxL(I + 1, J) * GeB(I, J - 1) + QxL(I, J) * GeB(I - 1, J - 1)) +
-                   -1.0 * (QBx(I + 1, J) * Ge(I, J - 1) + QBx(I, J) * Ge(I - 1, J - 1));
-        };
-        N = ((fx(i + 1, j) - fx(i + 1, j + 1)) + (fy(i + 1, j + 1) - fy(i, j + 1))) * a.nl_scale[lev];
+        const double* GB = a.GB + a.Gmap.off(lev);       // base Γ, this state's edge values
+        const double bw = i0 > 0 ? GB[o - 1] : gw, be = i0 < n1 - 1 ? GB[o + 1] : ge;
+        const double bs = j0 > 0 ? GB[o - P] : gs, bn = j0 < n2 - 1 ? GB[o + P] : gn;
+        Faces QB = faces(a.qB + (long long)lev * g.nq);
+        const double bx = 2.0 * a.q0Bx[lev], by = 2.0 * a.q0By[lev];
+        QB.w += bx; QB.e += bx; QB.s += by; QB.n += by;
+        N = (((Q.s * bs + QB.s * gs) - (Q.n * bn + QB.n * gn)) + ((Q.w * bw + QB.w * gw) - (Q.e * be + QB.e * ge))) *
+            a.nl_scale[lev];
     }
-
     // explicit viscous operator
-    const double gc = G[(long long)j0 * P + i0];
-    const double ge = (i0 + 1 < n1) ? G[(long long)j0 * P + i0 + 1] : 0.0;
-    const double gw = (i0 > 0) ? G[(long long)j0 * P + i0 - 1] : 0.0;
-    const double gn = (j0 + 1 < n2) ? G[(long long)(j0 + 1) * P + i0] : 0.0;
-    const double gs = (j0 > 0) ? G[(long long)(j0 - 1) * P + i0] : 0.0;
-    const double AG = gc + a.c_lap[lev] * ((((ge + gw) + gn) + gs) - 4.0 * gc);
-
-    // apply_bc!(rhsbc = 0, bc, fac) (mg-utils.jl:43-60)
-    double rbc = 0.0;
-    if (cb.rc) {
-        const double fac = a.fac_bc[lev];
-        if (j0 == 0) rbc += fac * cb.bot(i0 + 1);
-        if (j0 == n2 - 1) rbc += fac * cb.top(i0 + 1);
-        if (i0 == 0) rbc += fac * cb.left(j0 + 1);
-        if (i0 == n1 - 1) rbc += fac * cb.right(j0 + 1);
-    }
-    const long long o = a.Gmap.off(lev) + (long long)j0 * P + i0;
-    const double Np = a.Nprev[o];
-    a.Nnew[o] = N;
-    a.rhs[o] = ((AG + a.b1dt * N) + a.b2dt * Np) + rbc;
+    const double AG = gc + a.c_lap[lev] * ((((ze + zw) + zn) + zs) - 4.0 * gc);
+    const long long oo = a.Gmap.off(lev) + o;
+    const double Np = a.Nprev[oo];
+    a.Nnew[oo] = N;
+    a.rhs[oo] = ((AG + a.b1dt * N) + a.b2dt * Np) + rbc;
 }
 
 cudaError_t launch_trial_rhs(const Geom& g, const RhsArgs& a, cudaStream_t st) {
@@ -180,45 +168,56 @@ cudaError_t launch_coarsify(const Geom& g, double* G, SlabMap fine_map, SlabMap 
 // ψbc = get_bc!(ψ[lev+1]) (zero on the coarsest level).  Reproduces the
 // reference exactly, including the bottom row of x-fluxes reading ψbc[(B-1)+i]
 // (curl.jl:92), i.e. edge vertex i-2, where the top row reads vertex i-1.
-// One thread per flux element; blockIdx.y = batch × levels.
+// Each thread takes column I of kCurlRows rows and writes both fluxes, so a value
+// of ψ is loaded about twice instead of four times and the indices need no
+// division (one thread per flux element did both): per step of 512² x 5 levels
+// 34 -> 22 µs, of 1024² x 5 95 -> 41 µs (events; the latter moves 150 MB, 23 µs).
+// blockIdx.z = batch × levels.
 // ---------------------------------------------------------------------------
-__global__ void curl_kernel(CurlArgs a, Geom g) {
+constexpr int kCurlRows = 4;
+
+__global__ void __launch_bounds__(256) curl_kernel(CurlArgs a, Geom g) {
     pdl_wait();
     pdl_trigger();
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= g.nq) return;
-    const int y = blockIdx.y;
-    const int lev = a.psi_map.level(y);
-    const int bt = a.psi_map.batch(y);
+    const int I = blockIdx.x * blockDim.x + threadIdx.x + 1;                    // 1 … nx + 1
+    const int J0 = (blockIdx.y * blockDim.y + threadIdx.y) * kCurlRows + 1;     // rows J0 … of 1 … ny + 1
+    const int z = blockIdx.z;
+    const int lev = a.psi_map.level(z);
     const int nx = g.nx, ny = g.ny, P = g.P;
-    const double* psi = a.psi + a.psi_map.off(y);
-    CoarseBC eb;
-    eb.rc = (lev < a.mg - 1) ? a.coarse + a.coarse_map.off(y) : nullptr;
-    eb.P = P; eb.nx = nx; eb.ny = ny;
-    auto ps = [&](int I, int J) -> double { return psi[(long long)(J - 1) * P + (I - 1)]; };
-    double v;
-    if (e < g.nu) {
-        const int I = e % (nx + 1) + 1, J = e / (nx + 1) + 1;
-        if (I == 1) v = eb.left(J) - eb.left(J - 1);
-        else if (I == nx + 1) v = eb.right(J) - eb.right(J - 1);
-        else if (J == 1) v = ps(I - 1, 1) - eb.bot(I - 2);
-        else if (J == ny) v = eb.top(I - 1) - ps(I - 1, ny - 1);
-        else v = ps(I - 1, J) - ps(I - 1, J - 1);
-    } else {
-        const int f = e - g.nu;
-        const int I = f % nx + 1, J = f / nx + 1;
-        if (J == 1) v = eb.bot(I - 1) - eb.bot(I);
-        else if (J == ny + 1) v = eb.top(I - 1) - eb.top(I);
-        else if (I == 1) v = eb.left(J - 1) - ps(1, J - 1);
-        else if (I == nx) v = ps(nx - 1, J - 1) - eb.right(J - 1);
-        else v = ps(I - 1, J - 1) - ps(I, J - 1);
+    if (I > nx + 1 || J0 > ny + 1) return;
+    const double* psi = a.psi + a.psi_map.off(z);
+    double* qx = a.q + (long long)a.psi_map.batch(z) * a.q_bstride + (long long)(lev - a.q_lev0) * a.q_lstride;
+    double* qy = qx + g.nu;
+    if (I > 1 && I < nx && J0 > 1 && J0 + kCurlRows <= ny) {
+        const double* p = psi + (J0 - 2) * P + (I - 2);  // ψ(I−1, J0−1)
+        double w[kCurlRows + 1], e[kCurlRows];
+#pragma unroll
+        for (int r = 0; r <= kCurlRows; ++r) w[r] = p[r * P];
+#pragma unroll
+        for (int r = 0; r < kCurlRows; ++r) e[r] = p[r * P + 1];
+        const int ox = (I - 1) + (J0 - 1) * (nx + 1), oy = (I - 1) + (J0 - 1) * nx;
+#pragma unroll
+        for (int r = 0; r < kCurlRows; ++r) {
+            qx[ox + r * (nx + 1)] = w[r + 1] - w[r];
+            qy[oy + r * nx] = w[r] - e[r];
+        }
+        return;
     }
-    a.q[(long long)bt * a.q_bstride + (long long)(lev - a.q_lev0) * a.q_lstride + e] = v;
+    CurlAt at;
+    at.psi = psi; at.P = P; at.nx = nx; at.ny = ny;
+    at.eb.rc = (lev < a.mg - 1) ? a.coarse + a.coarse_map.off(z) : nullptr;
+    at.eb.P = P; at.eb.nx = nx; at.eb.ny = ny;
+    for (int r = 0; r < kCurlRows; ++r) {
+        const int J = J0 + r;
+        if (J <= ny) qx[(I - 1) + (J - 1) * (nx + 1)] = at.x(I, J);
+        if (J <= ny + 1 && I <= nx) qy[(I - 1) + (J - 1) * nx] = at.y(I, J);
+    }
 }
 
 cudaError_t launch_curl(const Geom& g, const CurlArgs& a, cudaStream_t st) {
-    dim3 grid((g.nq + 255) / 256, a.nlev * a.nbatch);
-    return launch_k(curl_kernel, grid, dim3(256), 0, st, a, g);
+    dim3 blk(32, 8);
+    dim3 grid((g.nx + 1 + 31) / 32, (g.ny + 1 + 8 * kCurlRows - 1) / (8 * kCurlRows), a.nlev * a.nbatch);
+    return launch_k(curl_kernel, grid, blk, 0, st, a, g);
 }
 
 // ---------------------------------------------------------------------------
