@@ -130,43 +130,67 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-// E (regT!, interface-coupling.jl:122-133) on (q + q0): one warp per force
-// component and batch member.  F[bt*F_bstride + kk*F_kstride].
+// E (regT!, interface-coupling.jl:122-133) on (q + q0) with q = C ψ of level 1
+// formed in place: one warp per force component and batch member, two ψ values
+// per flux of its 13×13 window, so the flux field itself is neither written nor
+// read (its curl launch took 7 µs of a 512² step, and 200 MB per 102 columns of
+// B on 400×200).  F[bt*F_bstride + kk*F_kstride].
 // A moving grid's base flux (MovingFlux, level 1) replaces the uniform q0x, q0y.
 // Moving bodies: F −= ub·h, the body-point velocity term of boundary_forces!
 // (timestepping.jl:174-186), when ub is set.
-__global__ void E_kernel(BodyDev b, Geom g, const double* __restrict__ q, long long q_stride, int nbatch,
-                         double q0x, double q0y, double* F, long long F_bstride, long long F_kstride,
-                         MovingFlux mv, const double* __restrict__ ub, double hub) {
-    pdl_wait();
-    pdl_trigger();
+// What bounds it is latency: the weights and indices of fixed bodies (FIXED) are
+// constants of the handle, so their loads are issued before the dependency wait.
+constexpr int kTaps = (169 + 31) / 32;   // window points per lane
+
+template <bool FIXED>
+__global__ void __launch_bounds__(256) E_kernel(BodyDev b, Geom g, const double* __restrict__ psi,
+                                                long long psi_bstride, int nbatch, double q0x, double q0y, double* F,
+                                                long long F_bstride, long long F_kstride, MovingFlux mv,
+                                                const double* __restrict__ ub, double hub) {
+    if constexpr (!FIXED) {
+        pdl_wait();
+        pdl_trigger();
+    }
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
-    if (warp >= b.nf * nbatch) return;
-    const int bt = warp / b.nf, kk = warp % b.nf;
+    const bool on = warp < b.nf * nbatch;
+    const int bt = on ? warp / b.nf : 0, kk = on ? warp % b.nf : 0;
     const int comp = kk / b.nb, k = kk % b.nb;
-    const double* qq = q + (long long)bt * q_stride;
     const int bx = b.bidx[k], by = b.bidx[b.nb + k];
     const double* w = b.w + (long long)kk * 169;
+    double wt[kTaps];
+#pragma unroll
+    for (int s = 0; s < kTaps; ++s) wt[s] = lane + 32 * s < 169 ? w[lane + 32 * s] : 0.0;
+    if constexpr (FIXED) {
+        pdl_wait();
+        pdl_trigger();
+    }
+    if (!on) return;
+    CurlAt at;
+    at.psi = psi + (long long)bt * psi_bstride;
+    at.P = g.P; at.nx = g.nx; at.ny = g.ny;
+    at.eb.rc = g.mg > 1 ? at.psi + g.S : nullptr;
+    at.eb.P = g.P; at.eb.nx = g.nx; at.eb.ny = g.ny;
     const double* mrow = mv.tab ? moving_row(mv) : nullptr;
     double acc = 0.0;
-    for (int t = lane; t < 169; t += 32) {
-        const int l = t / 13, m = t % 13;
-        const int I = bx + l - 6, J = by + m - 6;
-        double qv;
-        if (comp == 0)
-            qv = qq[(I - 1) + (long long)(J - 1) * (g.nx + 1)] + (mrow ? moving_q0x(mv, mrow, J, g.ny, mv.h) : q0x);
-        else
-            qv = qq[g.nu + (I - 1) + (long long)(J - 1) * g.nx] + (mrow ? moving_q0y(mv, mrow, I, g.nx, mv.h) : q0y);
-        acc += w[t] * qv;
+#pragma unroll
+    for (int s = 0; s < kTaps; ++s) {
+        const int t = lane + 32 * s;
+        if (t < 169) {
+            const int I = bx + t / 13 - 6, J = by + t % 13 - 6;
+            double qv;
+            if (comp == 0) qv = at.x(I, J) + (mrow ? moving_q0x(mv, mrow, J, g.ny, mv.h) : q0x);
+            else qv = at.y(I, J) + (mrow ? moving_q0y(mv, mrow, I, g.nx, mv.h) : q0y);
+            acc += wt[s] * qv;
+        }
     }
     acc = warp_sum(acc);
     if (ub) acc = acc - ub[kk] * hub;
     if (lane == 0) F[(long long)bt * F_bstride + (long long)kk * F_kstride] = acc;
 }
 
-cudaError_t launch_E(const Geom& g, const BodyDev& b, const double* q, long long q_stride, int nbatch,
-                     double q0x, double q0y, double* F, long long F_stride, cudaStream_t st,
+cudaError_t launch_E(const Geom& g, const BodyDev& b, const double* psi, long long psi_bstride, int nbatch,
+                     double q0x, double q0y, double* F, long long F_stride, bool fixed, cudaStream_t st,
                      const MovingFlux& mv, const double* ub, double hub) {
     // F_stride > 0: batch stride with unit component stride; F_stride < 0:
     // component stride |F_stride| with unit batch stride (columns of B).
@@ -174,26 +198,64 @@ cudaError_t launch_E(const Geom& g, const BodyDev& b, const double* q, long long
     const long long ks = F_stride > 0 ? 1 : -F_stride;
     const long long warps = (long long)b.nf * nbatch;
     const int blocks = (int)((warps * 32 + 255) / 256);
-    return launch_k(E_kernel, dim3(blocks), dim3(256), 0, st, b, g, q, q_stride, nbatch, q0x, q0y, F, bs, ks, mv, ub,
-                    hub);
+    return launch_k(fixed ? E_kernel<true> : E_kernel<false>, dim3(blocks), dim3(256), 0, st, b, g, psi, psi_bstride,
+                    nbatch, q0x, q0y, F, bs, ks, mv, ub, hub);
 }
 
-// y = A x, A row-major n×n: one warp per row (F̃b .= Binv*F̃b, timestepping.jl:160).
-__global__ void gemv_kernel(const double* __restrict__ A, const double* __restrict__ x, double* y, int n) {
-    pdl_wait();
-    pdl_trigger();
-    const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (row >= n) return;
-    const double* a = A + (long long)row * n;
+// y = A x, A row-major n×n (F̃b .= Binv*F̃b, timestepping.jl:160): WPR warps per
+// row, partial sums added in a fixed order.  One read of A bounds it (50 MB at
+// n = 2512, 7.7 µs); below that, latency, so with CONST (A not rewritten by the
+// step: fixed bodies) the thread's first kGemvPre values of A are loaded before
+// the dependency wait.
+constexpr int kGemvPre = 8;
+
+template <int WPR, bool CONST>
+__global__ void __launch_bounds__(256) gemv_kernel(const double* __restrict__ A, const double* __restrict__ x,
+                                                   double* y, int n) {
+    constexpr int RPB = 8 / WPR, T = 32 * WPR;           // rows per block, threads per row
+    __shared__ double part[8];
+    if constexpr (!CONST) {
+        pdl_wait();
+        pdl_trigger();
+    }
+    const int row = blockIdx.x * RPB + threadIdx.x / T, t = threadIdx.x % T;
+    const double* a = A + (long long)(row < n ? row : 0) * n;
+    double pre[kGemvPre];
+#pragma unroll
+    for (int s = 0; s < kGemvPre; ++s) pre[s] = t + s * T < n ? a[t + s * T] : 0.0;
+    if constexpr (CONST) {
+        pdl_wait();
+        pdl_trigger();
+    }
     double acc = 0.0;
-    for (int c = lane; c < n; c += 32) acc += a[c] * x[c];
+#pragma unroll
+    for (int s = 0; s < kGemvPre; ++s)
+        if (t + s * T < n) acc += pre[s] * x[t + s * T];
+#pragma unroll 8
+    for (int c = t + kGemvPre * T; c < n; c += T) acc += a[c] * x[c];
     acc = warp_sum(acc);
-    if (lane == 0) y[row] = acc;
+    if constexpr (WPR == 1) {
+        if (t == 0 && row < n) y[row] = acc;
+    } else {
+        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
+        __syncthreads();
+        if (t == 0 && row < n) {
+            double s = 0.0;
+#pragma unroll
+            for (int u = 0; u < WPR; ++u) s += part[(threadIdx.x >> 5) + u];
+            y[row] = s;
+        }
+    }
 }
 
-cudaError_t launch_gemv(const double* A, const double* x, double* y, int n, cudaStream_t st) {
-    return launch_k(gemv_kernel, dim3((n * 32 + 255) / 256), dim3(256), 0, st, A, x, y, n);
+// One warp per row up to n = 256 (eight values per lane); four above, where one
+// warp left a 25-step chain per lane at n = 804.
+cudaError_t launch_gemv(const double* A, const double* x, double* y, int n, bool constant, cudaStream_t st) {
+    if (n <= 256)
+        return launch_k(constant ? gemv_kernel<1, true> : gemv_kernel<1, false>, dim3((n + 7) / 8), dim3(256), 0, st, A,
+                        x, y, n);
+    return launch_k(constant ? gemv_kernel<4, true> : gemv_kernel<4, false>, dim3((n + 1) / 2), dim3(256), 0, st, A, x,
+                    y, n);
 }
 
 // update_stress! (timestepping.jl:330-354): fb = F̃b (h/dt) ./ ds,
@@ -202,7 +264,7 @@ cudaError_t launch_gemv(const double* A, const double* x, double* y, int n, cuda
 // One block; a non-finite CD/CL sets bit 0 of *status.
 __device__ __forceinline__ void stress_block(const BodyDev& b, const double* __restrict__ Fb, double h, double dt,
                                              double* hist, int hist_cap, int* counter, int* status) {
-    __shared__ double red[2][256];
+    __shared__ double red[2][8];
     const int step = *counter;
     const bool keep = step >= 0 && step < hist_cap;
     if (!keep && threadIdx.x == 0) atomicOr(status, 8);
@@ -215,18 +277,21 @@ __device__ __forceinline__ void stress_block(const BodyDev& b, const double* __r
             sx += ds * ((Fb[p] * hdt) / ds);
             sy += ds * ((Fb[b.nb + p] * hdt) / ds);
         }
-        red[0][threadIdx.x] = sx;
-        red[1][threadIdx.x] = sy;
-        __syncthreads();
-        for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-            if (threadIdx.x < s) {
-                red[0][threadIdx.x] += red[0][threadIdx.x + s];
-                red[1][threadIdx.x] += red[1][threadIdx.x + s];
-            }
-            __syncthreads();
+        sx = warp_sum(sx);
+        sy = warp_sum(sy);
+        if ((threadIdx.x & 31) == 0) {
+            red[0][threadIdx.x >> 5] = sx;
+            red[1][threadIdx.x >> 5] = sy;
         }
+        __syncthreads();
         if (threadIdx.x == 0) {
-            const double cd = 2.0 * red[0][0], cl = 2.0 * red[1][0];
+            double cd = 0.0, cl = 0.0;
+            for (int u = 0; u < 8; ++u) {
+                cd += red[0][u];
+                cl += red[1][u];
+            }
+            cd *= 2.0;
+            cl *= 2.0;
             if (keep) {
                 hist[((long long)step * 2 + 0) * b.nbodies + j] = cd;
                 hist[((long long)step * 2 + 1) * b.nbodies + j] = cl;
@@ -250,6 +315,8 @@ cudaError_t launch_stress(const BodyDev& b, const double* Fb, double h, double d
     return launch_k(stress_kernel, dim3(1), dim3(256), 0, st, b, Fb, h, dt, hist, hist_cap, counter, status);
 }
 
+// update_stress! and the projection source in one launch (both read only F̃b):
+// block 0 reduces CD/CL (and advances the step counter), the other blocks form
 // Γsrc = C'(E' F̃b) at the Γ points whose rot! stencil touches a regularised
 // flux point (timestepping.jl:217, curl.jl:22-34): Γ = (qx₁ − qx₂) +
 // (qy₁ − qy₂) over the point's four fluxes, each flux the sum over its sorted
@@ -257,47 +324,46 @@ cudaError_t launch_stress(const BodyDev& b, const double* Fb, double h, double d
 // the lanes take the contributors of all four fluxes (about 50 at one point
 // per h), with the signs of rot!, and a shuffle tree adds them in a fixed
 // order, so the result is deterministic (the reference adds sequentially;
-// the two agree to round-off).
-__device__ __forceinline__ void proj_src_warp(const BodyDev& b, const double* __restrict__ Fb, double* Gsrc, int p,
-                                              int lane) {
-    if (p >= b.n_src) return;
+// the two agree to round-off).  The lists and weights of fixed bodies are
+// constants: a lane's first contributor of each flux (lists of up to 32) is
+// looked up before the dependency wait, three dependent loads off the chain.
+__global__ void __launch_bounds__(256) stress_src_kernel(BodyDev b, const double* __restrict__ Fb, double h, double dt,
+                                                         double* hist, int hist_cap, int* counter, int* status,
+                                                         double* Gsrc) {
+    if (blockIdx.x == 0) {
+        pdl_wait();
+        pdl_trigger();
+        stress_block(b, Fb, h, dt, hist, hist_cap, counter, status);
+        return;
+    }
+    const int p = ((blockIdx.x - 1) * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    const bool on = p < b.n_src;
+    int next[4], end[4], kf[4];
+    double wf[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int row = on ? b.src_rows[4 * p + r] : -1;
+        next[r] = row < 0 ? 0 : b.et_ptr[row] + lane;
+        end[r] = row < 0 ? 0 : b.et_ptr[row + 1];
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const bool any = next[r] < end[r];
+        kf[r] = any ? b.et_k[next[r]] : 0;
+        wf[r] = any ? b.w[b.et_w[next[r]]] : 0.0;
+    }
+    pdl_wait();
+    pdl_trigger();
+    if (!on) return;
     double v = 0.0;
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-        const int row = b.src_rows[4 * p + r];
-        if (row < 0) continue;
-        double acc = 0.0;
-        for (int e = b.et_ptr[row] + lane; e < b.et_ptr[row + 1]; e += 32) acc += b.w[b.et_w[e]] * Fb[b.et_k[e]];
+        double acc = wf[r] * Fb[kf[r]];
+        for (int e = next[r] + 32; e < end[r]; e += 32) acc += b.w[b.et_w[e]] * Fb[b.et_k[e]];
         v += (r == 0 || r == 2) ? acc : -acc;
     }
     v = warp_sum(v);
     if (lane == 0) Gsrc[b.src_pts[p]] = v;
-}
-
-__global__ void proj_src_kernel(BodyDev b, const double* __restrict__ Fb, double* Gsrc) {
-    pdl_wait();
-    pdl_trigger();
-    proj_src_warp(b, Fb, Gsrc, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, threadIdx.x & 31);
-}
-
-cudaError_t launch_proj_src(const Geom& g, const BodyDev& b, const double* Fb, double* Gsrc, cudaStream_t st) {
-    if (b.n_src == 0) return cudaSuccess;
-    const long long threads = (long long)b.n_src * 32;
-    return launch_k(proj_src_kernel, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, st, b, Fb, Gsrc);
-}
-
-// update_stress! and the projection source in one launch (both read only F̃b):
-// block 0 reduces CD/CL (and advances the step counter), the other blocks
-// form C'E'F̃b, one warp per Γ point.
-__global__ void stress_src_kernel(BodyDev b, const double* __restrict__ Fb, double h, double dt, double* hist,
-                                  int hist_cap, int* counter, int* status, double* Gsrc) {
-    pdl_wait();
-    pdl_trigger();
-    if (blockIdx.x == 0) {
-        stress_block(b, Fb, h, dt, hist, hist_cap, counter, status);
-        return;
-    }
-    proj_src_warp(b, Fb, Gsrc, ((blockIdx.x - 1) * blockDim.x + threadIdx.x) >> 5, threadIdx.x & 31);
 }
 
 cudaError_t launch_stress_src(const BodyDev& b, const double* Fb, double h, double dt, double* hist, int hist_cap,

@@ -44,7 +44,6 @@ struct ibpm_handle {
     int cur = 0;                           // parity: G[cur], Nl[cur] hold the state
     double* psi = nullptr;                 // ψ, mg slabs
     double* q = nullptr;                   // q, (nq, mg) reference layout
-    double* qs = nullptr;                  // trial flux, level 1 only
     double* rhs = nullptr;                 // mg slabs of scratch
     double* Gsrc = nullptr;                // projection source, one slab, zero off-support
     double* F = nullptr;                   // E (qs + q0)
@@ -59,6 +58,8 @@ struct ibpm_handle {
     int* d_src_pts = nullptr; int* d_src_rows = nullptr; int* d_et_ptr = nullptr; int* d_et_k = nullptr;
     int* d_et_w = nullptr; int* d_et_flux = nullptr;
     BodyDev body{};
+    int win_y0 = 0, win_y1 = 0;            // slab rows of ψ that E reads (fixed bodies), [y0, y1)
+    bool win_inside = false;               // … none of them through the level's edge values
     // per-step outputs
     double* hist = nullptr; int hist_cap = 0;
     double* pin_hist = nullptr;            // page-locked host mirror of hist (the advance read-back)
@@ -97,7 +98,7 @@ struct ibpm_handle {
     double* d_ub = nullptr;                // body-point velocities (nb, 2)
     int* d_bbox = nullptr;                 // min/max body_idx of the step
     double* btab = nullptr; int btab_cap = 0;
-    double *bGB = nullptr, *bPB = nullptr, *bQB = nullptr, *bwork = nullptr;  // per-step B rebuild
+    double *bGB = nullptr, *bPB = nullptr, *bwork = nullptr;  // per-step B rebuild
     int* binfo = nullptr;
     // discrete adjoint (allocated by the first ibpm_adjoint_run)
     int adj_k = 0, adj_ncp = 0, adj_nsteps = 0;
@@ -337,9 +338,11 @@ static int per_member(ibpm_handle* h, F fn) {
 // F̃b = B⁻¹ F, then update_stress! and the projection source.
 static int forces_and_src(ibpm_handle* h) {
     const Geom& g = h->g;
-    LAUNCH(K_E, 16.0 * 169 * h->nf, launch_E(g, h->body, h->qs, 0, 1, h->q0x[0], h->q0y[0], h->F, h->nf, h->st, mv_of(h),
-                    h->bodies_moving ? h->d_ub : nullptr, h->h));
-    LAUNCH(K_GEMV, 8.0 * h->nf * (h->nf + 2.0), launch_gemv(h->Binv, h->F, h->Fb, h->nf, h->st));
+    const bool fixed = !h->bodies_moving;
+    LAUNCH(K_E, 16.0 * 169 * h->nf,
+           launch_E(g, h->body, h->psi, 0, 1, h->q0x[0], h->q0y[0], h->F, h->nf, fixed, h->st, mv_of(h),
+                    fixed ? nullptr : h->d_ub, h->h));
+    LAUNCH(K_GEMV, 8.0 * h->nf * (h->nf + 2.0), launch_gemv(h->Binv, h->F, h->Fb, h->nf, fixed, h->st));
     return stress_and_src(h);
 }
 
@@ -367,10 +370,10 @@ static RhsArgs rhs_args(const ibpm_handle* h, int p) {
 // vort2flux! (curl.jl:133-165) on `nbatch` independent fields G (slab-major,
 // batch stride bstride), level by level as the reference: coarsify chain,
 // Δ⁻¹ solves from the coarsest level inwards with the edge values of the next
-// coarser ψ, then q = curl ψ on levels [qlev0, qlev0 + qnlev) into q (nq per
-// level, batch stride q_bstride).
+// coarser ψ, then q = curl ψ on levels < qnlev (none when only ψ is wanted)
+// into q (nq per level, batch stride q_bstride).
 static int vort2flux(ibpm_handle* h, double* G, double* psi, long long bstride, int nbatch, double* q,
-                     long long q_bstride, int qlev0, int qnlev) {
+                     long long q_bstride, int qnlev) {
     const Geom& g = h->g;
     const int mg = g.mg;
     for (int lev = 1; lev < mg; ++lev)
@@ -383,10 +386,11 @@ static int vort2flux(ibpm_handle* h, double* G, double* psi, long long bstride, 
                          levmap(g, lev + 1, 1, bstride));
         if (rc) return rc;
     }
+    if (qnlev < 1) return IBPM_OK;
     CurlArgs ca{};
-    ca.psi = psi; ca.psi_map = levmap(g, qlev0, qnlev, bstride);
-    ca.coarse = psi; ca.coarse_map = levmap(g, qlev0 + 1, qnlev, bstride);
-    ca.q = q; ca.q_bstride = q_bstride; ca.q_lstride = g.nq; ca.q_lev0 = qlev0;
+    ca.psi = psi; ca.psi_map = levmap(g, 0, qnlev, bstride);
+    ca.coarse = psi; ca.coarse_map = levmap(g, 1, qnlev, bstride);
+    ca.q = q; ca.q_bstride = q_bstride; ca.q_lstride = g.nq; ca.q_lev0 = 0;
     ca.nlev = qnlev; ca.nbatch = nbatch; ca.mg = mg;
     LAUNCH(K_CURL, 8.0 * ((double)g.n1 * g.n2 + g.nq) * qnlev * nbatch, launch_curl(g, ca, h->st));
     return IBPM_OK;
@@ -532,10 +536,12 @@ static int curl_levels(ibpm_handle* h, double* q, int qnlev) {
 }
 
 // vort2flux! (FP64) of the handle's field G into h->psi (levels < nfull; the
-// coarser ones are left as they were) and q (levels < qnlev < nfull).  The
-// trial vort2flux! of a step needs only the level-1 flux, hence ψ of levels 1
-// and 2; the final one recomputes every level.
-static int vort2flux_bt(ibpm_handle* h, double* G, double* q, int qnlev, int nfull) {
+// coarser ones are left as they were) and q (levels < qnlev <= nfull; none
+// when only ψ is wanted); of a single level only its rows [y0, y1) where y1 > 0.
+// E of the trial vort2flux! reads ψ of level 1 around the bodies, and of level
+// 2 where a body's window meets the level's edge (trial_window); the final
+// vort2flux! recomputes every level.
+static int vort2flux_bt(ibpm_handle* h, double* G, double* q, int qnlev, int nfull, int y0 = 0, int y1 = 0) {
     const Geom& g = h->g;
     const int mg = g.mg, ns = h->gsim;
     const long long bs = g.S * mg;
@@ -555,9 +561,10 @@ static int vort2flux_bt(ibpm_handle* h, double* G, double* q, int qnlev, int nfu
     SlabMap part = levmap(g, 0, nfull, bs);
     XPassArgs c{};
     c.in = h->rhs; c.in2 = h->btY; c.in_map = part; c.in2_map = part; c.out = h->psi; c.out_map = part;
-    c.nslabs = nfull * ns; c.line0 = 0; c.line1 = g.n2; c.load = XLOAD_SUM; c.emit = XEMIT_STORE;
-    LAUNCH(K_DSTX, 24.0 * slab * nfull * ns, launch_dst_x(g, h->px, c, h->st));
-    return curl_levels(h, q, qnlev);
+    c.nslabs = nfull * ns; c.line0 = y1 > 0 ? y0 : 0; c.line1 = y1 > 0 ? y1 : g.n2;
+    c.load = XLOAD_SUM; c.emit = XEMIT_STORE;
+    LAUNCH(K_DSTX, 24.0 * slab * nfull * ns * (c.line1 - c.line0) / g.n2, launch_dst_x(g, h->px, c, h->st));
+    return qnlev > 0 ? curl_levels(h, q, qnlev) : IBPM_OK;
 }
 
 // vort2flux! of FP32_REFINED: `nsw` sweeps ψ ← ψ + d, the corrections d of
@@ -608,6 +615,25 @@ static int trial_rhs(ibpm_handle* h, int p) {
     return IBPM_OK;
 }
 
+// The part of ψ that E reads after the trial vort2flux! of the FP64 step: for
+// fixed bodies inside the level, the rows of level 1 around them (of every
+// member of the group being captured); else levels 1 and 2.  At 512² x 5 with a
+// unit cylinder this is 140 of 511 rows: the last x-pass takes 6 µs instead of
+// 10, the edge part's y-solve one level instead of two.
+struct TrialWindow { int nfull, y0, y1; };
+static TrialWindow trial_window(const ibpm_handle* h) {
+    TrialWindow w{std::min(2, h->g.mg), 0, 0};
+    if (h->bodies_moving) return w;
+    int y0 = h->g.n2, y1 = 0;
+    for (int i = 0; i < h->gsim; ++i) {
+        const ibpm_handle* m = h->gsim > 1 ? h->gmem[i] : h;
+        if (!m->win_inside) return w;
+        y0 = std::min(y0, m->win_y0);
+        y1 = std::max(y1, m->win_y1);
+    }
+    return TrialWindow{1, y0, y1};
+}
+
 // One step, reading the state from parity p and leaving it in parity p^1.
 static int enqueue_step_fp64(ibpm_handle* h, int p) {
     const Geom& g = h->g;
@@ -621,8 +647,9 @@ static int enqueue_step_fp64(ibpm_handle* h, int p) {
     SlabMap all = levmap(g, 0, mg);
     rc = poisson(h, h->rhs, all, h->rhs, all, Gnew, all, mg * ns, SPEC_AINV, XEMIT_STORE);
     if (rc) return rc;
-    rc = h->bt ? vort2flux_bt(h, Gnew, h->qs, 1, std::min(2, mg))  // only the level-1 trial flux is read
-               : vort2flux(h, Gnew, h->psi, g.S * mg, ns, h->qs, qb, 0, 1);
+    const TrialWindow tw = trial_window(h);
+    rc = h->bt ? vort2flux_bt(h, Gnew, nullptr, 0, tw.nfull, tw.y0, tw.y1)
+               : vort2flux(h, Gnew, h->psi, g.S * mg, ns, nullptr, 0, 0);
     if (rc) return rc;
     // --- boundary_forces! (timestepping.jl:154-163), update_stress! (:330-354)
     if ((rc = per_member(h, forces_and_src))) return rc;
@@ -631,7 +658,7 @@ static int enqueue_step_fp64(ibpm_handle* h, int p) {
     rc = poisson(h, h->Gsrc, one, h->rhs, one, Gnew, one, ns, SPEC_AINV, XEMIT_SUB);
     if (rc) return rc;
     // --- vort2flux!(state.ψ, state.q, state.Γ) (timestepping.jl:64)
-    return h->bt ? vort2flux_bt(h, Gnew, h->q, mg, mg) : vort2flux(h, Gnew, h->psi, g.S * mg, ns, h->q, qb, 0, mg);
+    return h->bt ? vort2flux_bt(h, Gnew, h->q, mg, mg) : vort2flux(h, Gnew, h->psi, g.S * mg, ns, h->q, qb, mg);
 }
 
 // ---------------------------------------------------------------------------
@@ -719,8 +746,8 @@ static int enqueue_step_refined(ibpm_handle* h, int p, int nsw) {
     // cycle's CL amplitude by 3e-6, against 2.5e-7 this way, and it cost more.
     // The final vort2flux! refines from it: levels it did not complete keep
     // the previous step's ψ and take a whole step's correction there.
-    rc = h->bt ? vort2flux_bt(h, Gnew, h->qs, 1, std::min(2, mg))
-               : vort2flux(h, Gnew, h->psi, g.S * mg, ns, h->qs, (long long)g.nq * mg, 0, 1);
+    rc = h->bt ? vort2flux_bt(h, Gnew, nullptr, 0, std::min(2, mg))
+               : vort2flux(h, Gnew, h->psi, g.S * mg, ns, nullptr, 0, 0);
     if (rc) return rc;
     // --- boundary_forces! and update_stress! (FP64)
     if ((rc = per_member(h, forces_and_src))) return rc;
@@ -757,9 +784,9 @@ static int enqueue_body_update(ibpm_handle* h) {
         SlabMap l0 = levmap(g, 0, 1, bstride);
         int rc = poisson(h, h->bGB, l0, h->bGB, l0, h->bGB, l0, R, SPEC_AINV, XEMIT_STORE);
         if (rc) return rc;
-        rc = vort2flux(h, h->bGB, h->bPB, bstride, R, h->bQB, g.nq, 0, 1);
+        rc = vort2flux(h, h->bGB, h->bPB, bstride, R, nullptr, 0, 0);
         if (rc) return rc;
-        LAUNCH(K_E, 16.0 * 169 * R, launch_E(g, h->body, h->bQB, g.nq, R, 0.0, 0.0, h->Binv + c0, -(long long)nf, h->st));
+        LAUNCH(K_E, 16.0 * 169 * R, launch_E(g, h->body, h->bPB, bstride, R, 0.0, 0.0, h->Binv + c0, -(long long)nf, false, h->st));
     }
     LAUNCH(K_GEMV, 8.0 * 4.0 * nf * nf, launch_gj_inverse(h->Binv, nf, h->bwork, h->binfo, h->st));
     LAUNCH(K_GEMV, 8.0, launch_info_to_status(h->binfo, h->status, h->st));
@@ -790,6 +817,15 @@ static int build_coupling(ibpm_handle* h, const ibpm_problem_desc* d) {
         if (bx - 6 < 1 || bx + 6 > g.nx || by - 6 < 1 || by + 6 > g.ny)
             return fail(h, IBPM_ERR_INVALID, "body point " + std::to_string(k) +
                                                  ": the 13x13 regularisation stencil leaves the finest grid");
+    }
+    // E reads q = C ψ at fluxes (bidx ± 6): ψ of slab rows by − 8 … by + 5, and
+    // the edge values where a window meets the first or last flux of a row or column
+    {
+        const auto mx = std::minmax_element(bidx.begin(), bidx.begin() + nb);
+        const auto my = std::minmax_element(bidx.begin() + nb, bidx.end());
+        h->win_y0 = std::max(0, *my.first - 8);
+        h->win_y1 = std::min(g.n2, *my.second + 6);
+        h->win_inside = *mx.first - 6 >= 2 && *mx.second + 6 <= g.nx - 1 && *my.first - 6 >= 2 && *my.second + 6 <= g.ny - 1;
     }
     // E' as CSR over touched flux points, contributors in ascending component order.
     std::map<int, std::vector<std::pair<int, int>>> rows;  // flux index -> (kk, widx)
@@ -870,14 +906,14 @@ static int build_binv(ibpm_handle* h) {
     const Geom& g = h->g;
     const int nf = h->nf, mg = g.mg;
     const int chunk = std::min(nf, kBChunk);
-    double *GB = nullptr, *PB = nullptr, *QB = nullptr, *work = nullptr;
+    double *GB = nullptr, *PB = nullptr, *work = nullptr;
     int* info = nullptr;
     int rc;
     const long long bstride = g.S * mg;
     if ((rc = dalloc(h, &GB, (size_t)bstride * chunk)) || (rc = dalloc(h, &PB, (size_t)bstride * chunk)) ||
-        (rc = dalloc(h, &QB, (size_t)g.nq * chunk)) || (rc = dalloc(h, &work, gj_work_doubles(nf))) ||
+        (rc = dalloc(h, &work, gj_work_doubles(nf))) ||
         (rc = dalloc(h, &info, 1))) {
-        cudaFree(GB); cudaFree(PB); cudaFree(QB); cudaFree(work); cudaFree(info);
+        cudaFree(GB); cudaFree(PB); cudaFree(work); cudaFree(info);
         return rc;
     }
     // B at create is built with the single-level (latency) plan on every
@@ -887,7 +923,7 @@ static int build_binv(ibpm_handle* h) {
     h->px.planN = h->px.plan1;
     auto cleanup = [&]() {
         h->px.planN = planN;
-        cudaFree(GB); cudaFree(PB); cudaFree(QB); cudaFree(work); cudaFree(info);
+        cudaFree(GB); cudaFree(PB); cudaFree(work); cudaFree(info);
     };
     for (int c0 = 0; c0 < nf && rc == IBPM_OK; c0 += chunk) {
         const int R = std::min(chunk, nf - c0);
@@ -896,9 +932,9 @@ static int build_binv(ibpm_handle* h) {
         SlabMap l0 = levmap(g, 0, 1, bstride);
         rc = poisson(h, GB, l0, GB, l0, GB, l0, R, SPEC_AINV, XEMIT_STORE);
         if (rc) break;
-        rc = vort2flux(h, GB, PB, bstride, R, QB, g.nq, 0, 1);  // level-1 flux of each column
+        rc = vort2flux(h, GB, PB, bstride, R, nullptr, 0, 0);  // ψ of each column
         if (rc) break;
-        if (launch_E(g, h->body, QB, g.nq, R, 0.0, 0.0, h->Binv + c0, -(long long)nf, h->st) != cudaSuccess) {
+        if (launch_E(g, h->body, PB, bstride, R, 0.0, 0.0, h->Binv + c0, -(long long)nf, false, h->st) != cudaSuccess) {
             rc = IBPM_ERR_CUDA;
             break;
         }
@@ -931,7 +967,7 @@ static void free_handle(ibpm_handle* h) {
         if (p) cudaFree(p);
     if (h->mtab) cudaFree(h->mtab);
     for (void* p : {(void*)h->d_x0, (void*)h->d_ub, (void*)h->d_bbox, (void*)h->btab, (void*)h->bGB, (void*)h->bPB,
-                    (void*)h->bQB, (void*)h->bwork, (void*)h->binfo})
+                    (void*)h->bwork, (void*)h->binfo})
         if (p) cudaFree(p);
     if (h->GB) cudaFree(h->GB);
     if (h->qB) cudaFree(h->qB);
@@ -940,7 +976,7 @@ static void free_handle(ibpm_handle* h) {
                    h->qsb, h->Ft, h->Fbar, h->bcc, h->bcv, h->q0part, h->stepw, h->adj_n, h->wd, h->tapeFb,
                    h->tapeq1, h->gxb};
     for (void* p : adj) if (p) cudaFree(p);
-    void* ptrs[] = {h->G[0], h->G[1], h->Nl[0], h->Nl[1], h->psi, h->q, h->qs, h->rhs, h->Gsrc, h->F, h->Fb,
+    void* ptrs[] = {h->G[0], h->G[1], h->Nl[0], h->Nl[1], h->psi, h->q, h->rhs, h->Gsrc, h->F, h->Fb,
                     h->Binv, h->nonlin1_shadow, h->d_xb, h->d_ds, h->d_bidx, h->d_w, h->d_body_start,
                     h->d_src_pts, h->d_src_rows, h->d_et_ptr, h->d_et_k, h->d_et_w, h->d_et_flux, h->hist,
                     h->counter, h->status};
@@ -1008,7 +1044,7 @@ static int create_impl(ibpm_handle* h, const ibpm_problem_desc* d) {
     int rc;
     if ((rc = dalloc(h, &h->G[0], slabs)) || (rc = dalloc(h, &h->G[1], slabs)) || (rc = dalloc(h, &h->Nl[0], slabs)) ||
         (rc = dalloc(h, &h->Nl[1], slabs)) || (rc = dalloc(h, &h->psi, slabs)) ||
-        (rc = dalloc(h, &h->q, (size_t)g.nq * g.mg)) || (rc = dalloc(h, &h->qs, (size_t)g.nq * g.mg)) ||
+        (rc = dalloc(h, &h->q, (size_t)g.nq * g.mg)) ||
         (rc = dalloc(h, &h->rhs, slabs)) || (rc = dalloc(h, &h->Gsrc, g.S)) || (rc = dalloc(h, &h->F, h->nf)) ||
         (rc = dalloc(h, &h->Fb, h->nf)) || (rc = dalloc(h, &h->Binv, (size_t)h->nf * h->nf)) ||
         (rc = dalloc(h, &h->nonlin1_shadow, slabs)) || (rc = dalloc(h, &h->counter, 1)) ||
@@ -1017,7 +1053,6 @@ static int create_impl(ibpm_handle* h, const ibpm_problem_desc* d) {
     for (double* p : {h->G[0], h->G[1], h->Nl[0], h->Nl[1], h->psi, h->rhs, h->nonlin1_shadow})
         CK(cudaMemsetAsync(p, 0, sizeof(double) * slabs, h->st));
     CK(cudaMemsetAsync(h->q, 0, sizeof(double) * g.nq * g.mg, h->st));
-    CK(cudaMemsetAsync(h->qs, 0, sizeof(double) * g.nq * g.mg, h->st));
     CK(cudaMemsetAsync(h->Gsrc, 0, sizeof(double) * g.S, h->st));
     CK(cudaMemsetAsync(h->Fb, 0, sizeof(double) * h->nf, h->st));
     CK(cudaMemsetAsync(h->status, 0, sizeof(int), h->st));
@@ -1363,7 +1398,7 @@ extern "C" int ibpm_set_motion_function(ibpm_handle* h) {
     int rc;
     if ((rc = dalloc(h, &h->d_x0, 2 * h->nb)) || (rc = dalloc(h, &h->d_ub, 2 * h->nb)) ||
         (rc = dalloc(h, &h->d_bbox, 4)) || (rc = dalloc(h, &h->bGB, (size_t)bstride * chunk)) ||
-        (rc = dalloc(h, &h->bPB, (size_t)bstride * chunk)) || (rc = dalloc(h, &h->bQB, (size_t)g.nq * chunk)) ||
+        (rc = dalloc(h, &h->bPB, (size_t)bstride * chunk)) ||
         (rc = dalloc(h, &h->bwork, gj_work_doubles(nf))) || (rc = dalloc(h, &h->binfo, 1)))
         return rc;
     // the reference configuration x0 is the body as created (RigidBody.x0)
@@ -1410,7 +1445,7 @@ extern "C" int ibpm_vort2flux(ibpm_handle* h) {
     if (!h) return IBPM_ERR_INVALID;
     CK(cudaSetDevice(h->device));
     int rc = h->bt ? vort2flux_bt(h, h->G[h->cur], h->q, h->g.mg, h->g.mg)
-                   : vort2flux(h, h->G[h->cur], h->psi, h->g.S * h->g.mg, 1, h->q, 0, 0, h->g.mg);
+                   : vort2flux(h, h->G[h->cur], h->psi, h->g.S * h->g.mg, 1, h->q, 0, h->g.mg);
     if (rc) return rc;
     CK(cudaStreamSynchronize(h->st));
     return IBPM_OK;
@@ -2034,7 +2069,7 @@ static void batch_free_graphs(ibpm_batch* b) {
 
 // The step fields of a group's members moved into arenas, member after member
 // with the strides the shared launches assume: mg slabs for every slab field
-// (Gsrc and Pp included, though they use one), nq·mg for q and qs, and the
+// (Gsrc and Pp included, though they use one), nq·mg for q, and the
 // boundary-transfer vectors at their per-simulation sizes.  The content is
 // kept; each member then points into the arenas.
 template <class T, class F>
@@ -2068,7 +2103,7 @@ static void forget_arena_fields(ibpm_handle* h, const BatchGroup& gr) {
             if (c && c >= a.first && c < a.first + a.second) { p = nullptr; return; }
     };
     drop(h->G[0]); drop(h->G[1]); drop(h->Nl[0]); drop(h->Nl[1]);
-    drop(h->psi); drop(h->q); drop(h->qs); drop(h->rhs); drop(h->Gsrc); drop(h->Pp);
+    drop(h->psi); drop(h->q); drop(h->rhs); drop(h->Gsrc); drop(h->Pp);
     drop(h->T32);
     drop(h->btY); drop(h->btS); drop(h->btE); drop(h->btP);
     drop(h->btY32);
@@ -2100,7 +2135,6 @@ static int batch_make_group(ibpm_batch* b, const std::vector<ibpm_handle*>& mem)
     rd([](ibpm_handle* h) -> double*& { return h->Gsrc; }, slabs, (size_t)g.S);
     rd([](ibpm_handle* h) -> double*& { return h->Pp; }, slabs, (size_t)g.S);
     rd([](ibpm_handle* h) -> double*& { return h->q; }, nq, nq);
-    rd([](ibpm_handle* h) -> double*& { return h->qs; }, nq, nq);
     rf([](ibpm_handle* h) -> float*& { return h->T32; }, slabs, slabs);
     rd([](ibpm_handle* h) -> double*& { return h->btY; }, slabs, slabs);
     rf([](ibpm_handle* h) -> float*& { return h->btY32; }, slabs, slabs);

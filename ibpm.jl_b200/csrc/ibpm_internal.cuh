@@ -440,10 +440,11 @@ struct BodyDev {
 };
 cudaError_t launch_weights(const Geom& g, double h, double offx, double offy,
                            const BodyDev& b, cudaStream_t st);
-cudaError_t launch_E(const Geom& g, const BodyDev& b, const double* q, long long q_stride,
-                     int nbatch, double q0x, double q0y, double* F, long long F_stride,
-                     cudaStream_t st, const MovingFlux& mv = MovingFlux{}, const double* ub = nullptr,
-                     double hub = 0.0);
+// E (C ψ + q0) of level 1 from ψ (its slab, the next level's behind it); fixed:
+// the body's weights and indices are not rewritten by earlier launches.
+cudaError_t launch_E(const Geom& g, const BodyDev& b, const double* psi, long long psi_bstride, int nbatch,
+                     double q0x, double q0y, double* F, long long F_stride, bool fixed, cudaStream_t st,
+                     const MovingFlux& mv = MovingFlux{}, const double* ub = nullptr, double hub = 0.0);
 // Moving bodies (MotionFunction): kinematics from the step's motion-table row,
 // the projection source in gather form, and the singular-B flag.
 cudaError_t launch_kinematics(const Geom& g, const BodyDev& b, const double* x0, const double* tab, const int* step,
@@ -452,14 +453,13 @@ cudaError_t launch_kinematics(const Geom& g, const BodyDev& b, const double* x0,
 cudaError_t launch_proj_src_moving(const Geom& g, const BodyDev& b, const double* Fb, const int* bbox, double* Gsrc,
                                    cudaStream_t st);
 cudaError_t launch_info_to_status(const int* info, int* status, cudaStream_t st);
-cudaError_t launch_gemv(const double* A, const double* x, double* y, int n, cudaStream_t st);
+// y = A x; constant: A is not rewritten by earlier launches.
+cudaError_t launch_gemv(const double* A, const double* x, double* y, int n, bool constant, cudaStream_t st);
 // The force history holds hist_cap steps: a step past it writes nothing and
 // sets bit 3 of *status.
 cudaError_t launch_stress(const BodyDev& b, const double* Fb, double h, double dt,
                           double* hist, int hist_cap, int* counter, int* status, cudaStream_t st);
-cudaError_t launch_proj_src(const Geom& g, const BodyDev& b, const double* Fb, double* Gsrc,
-                            cudaStream_t st);
-// launch_stress and launch_proj_src in one launch (fixed bodies)
+// launch_stress and the projection source C'E'F̃b in one launch (fixed bodies)
 cudaError_t launch_stress_src(const BodyDev& b, const double* Fb, double h, double dt, double* hist, int hist_cap,
                               int* counter, int* status, double* Gsrc, cudaStream_t st);
 cudaError_t launch_unit_src(const Geom& g, const BodyDev& b, int col0, int ncol, double* G,
