@@ -31,6 +31,7 @@
 // free of bank conflicts.
 #pragma once
 
+#include <algorithm>
 #include <type_traits>
 
 #include "ibpm_internal.cuh"
@@ -73,6 +74,13 @@ __host__ __device__ constexpr int ct_tp(int N, int PL = 0) {
     int t = (((ct_fine(N, PL) ? N / 4 : N / 8) + 31) / 32) * 32;
     return t < 32 ? 32 : t;
 }
+// Lengths whose x-pass runs as resident CTAs looping over line pairs.  Their
+// stage indices (odd radices) do not reduce to constants; in the loop they are
+// invariants, formed once and before the dependency wait: the step of 400x200 x
+// 5 levels takes 115 µs instead of 130, of 384x192 x 5 111 instead of 120, of
+// 192² x 4 84 instead of 88.  Powers of two have constant offsets and lose 3-5%
+// to the invariants' registers, 768² 2%.
+__host__ __device__ constexpr bool ct_loop(int N) { return (N & (N - 1)) != 0 && N < 768; }
 __host__ __device__ constexpr int ct_pad(int i) { return i + (i >> 3); }
 __host__ __device__ constexpr int ct_buf(int N) { return ct_pad(N) + 8; }  // + scan scratch
 
@@ -219,19 +227,35 @@ template <int TP, int G> __device__ __forceinline__ void gsync(int gid) {
     }
 }
 
+// Whether pad(i + r·step) − pad(i) does not depend on i, for the i of a stage:
+// steps of whole pad periods never carry, and a step dividing the period does
+// not where i mod 8 stays below the step (or below 8 less the largest r·step).
+// The index arithmetic is then one base per butterfly and constants; without
+// it, it was about half of a transform's instructions.
+__host__ __device__ constexpr bool ct_whole(int step) { return step % 8 == 0; }
+__host__ __device__ constexpr bool ct_out_const(int R, int Ns) {
+    return ct_whole(Ns) || (8 % Ns == 0 && (Ns * R) % 8 == 0) || (Ns == 1 && 8 % R == 0);
+}
+__host__ __device__ constexpr int ct_off(int d) { return d + (d >> 3); }
+
 template <int N, int TP, int G, int R, int Ns, int TWOFF, class T>
 __device__ __forceinline__ void fft_stage(cplx_t<T>* buf, const cplx_t<T>* W, int tid, int gid) {
     using V = cplx_t<T>;
     constexpr int nb = N / R;
     constexpr int QM = (nb + TP - 1) / TP;
     constexpr bool exact = (QM * TP == nb);
+    static_assert(TP % 8 == 0, "a group is whole pad periods");
     V v[QM][R];
+    const V* in = buf + ct_pad(tid);
 #pragma unroll
     for (int q = 0; q < QM; ++q) {
         const int b = tid + q * TP;
         if (exact || b < nb) {
 #pragma unroll
-            for (int r = 0; r < R; ++r) v[q][r] = buf[ct_pad(b + r * nb)];
+            for (int r = 0; r < R; ++r) {
+                if constexpr (ct_whole(nb)) v[q][r] = in[ct_off(q * TP + r * nb)];
+                else v[q][r] = buf[ct_pad(b + r * nb)];
+            }
         }
     }
     gsync<TP, G>(gid);
@@ -246,8 +270,12 @@ __device__ __forceinline__ void fft_stage(cplx_t<T>* buf, const cplx_t<T>* W, in
             }
             dft_t<R, T>::run(v[q]);
             const int base = (b - k) * R + k;
+            V* out = buf + ct_pad(base);
 #pragma unroll
-            for (int r = 0; r < R; ++r) buf[ct_pad(base + r * Ns)] = v[q][r];
+            for (int r = 0; r < R; ++r) {
+                if constexpr (ct_out_const(R, Ns)) out[ct_off(r * Ns)] = v[q][r];
+                else buf[ct_pad(base + r * Ns)] = v[q][r];
+            }
         }
     }
     gsync<TP, G>(gid);
@@ -262,34 +290,49 @@ __device__ __forceinline__ void fft_stages(cplx_t<T>* buf, const cplx_t<T>* W, i
     }
 }
 
-// Pre-processing: buf[m] = y_m from load(m-1) = (a_{m-1}, b_{m-1}).
-template <int N, int TP, class T, class Load>
-__device__ __forceinline__ void dst_pre(cplx_t<T>* buf, const T* s, int tid, Load load) {
+// Pre-processing: buf[m] = y_m from load(m-1) = (a_{m-1}, b_{m-1}).  fix(i, v)
+// completes a loaded value (the edge terms).  The loads carry no branch, so all
+// of a thread's are in flight together: the thread of slot m = 0 (y_0 = 0) takes
+// m = N/2 instead, and indices past the end are clamped.
+template <int N, int TP, class T, class Load, class Fix>
+__device__ __forceinline__ void dst_pre(cplx_t<T>* buf, const T* s, int tid, Load load, Fix fix) {
     using V = cplx_t<T>;
     constexpr int half = N >> 1;
-    constexpr int IT = (half + TP) / TP;  // m = tid + it·TP covers 0 … half
+    constexpr int IT = (half + TP - 1) / TP;  // m = tid + it·TP covers 0 … half − 1
+    constexpr bool exact = IT * TP == half;
     V fm[IT], fn[IT];
+    V* const up = buf + ct_pad(tid);          // slots m = tid + it·TP
+    V* const dn = buf + ct_pad(N - tid);      // slots N − m
+    auto idx = [&](int it, int& i, int& j) {
+        int m = tid + it * TP;
+        if (!exact && m >= half) m = half - 1;
+        if (m == 0) m = half;
+        i = m - 1;
+        j = N - m - 1;
+    };
 #pragma unroll
-    for (int it = 0; it < IT; ++it) {  // issue every load before using any
-        const int m = tid + it * TP;
-        if (m >= 1 && m <= half) {
-            fm[it] = load(m - 1);
-            if (m < half) fn[it] = load(N - m - 1);
-        }
+    for (int it = 0; it < IT; ++it) {
+        int i, j;
+        idx(it, i, j);
+        fm[it] = load(i);
+        fn[it] = load(j);
     }
 #pragma unroll
     for (int it = 0; it < IT; ++it) {
         const int m = tid + it * TP;
-        if (m == 0) {
+        int i, j;
+        idx(it, i, j);
+        fm[it] = fix(i, fm[it]);
+        if (it == 0 && m == 0) {
             buf[0] = V{T(0), T(0)};
-        } else if (m == half) {  // sin(π/2) = 1
-            buf[ct_pad(m)] = V{T(2) * fm[it].x, T(2) * fm[it].y};
-        } else if (m < half) {
+            buf[ct_pad(half)] = V{T(2) * fm[it].x, T(2) * fm[it].y};  // sin(π/2) = 1
+        } else if (exact || m < half) {
+            fn[it] = fix(j, fn[it]);
             const T sm = s[m];
             const V sum = cadd(fm[it], fn[it]), dif = csub(fm[it], fn[it]);
             const V ys = V{sm * sum.x, sm * sum.y};
-            buf[ct_pad(m)] = V{ys.x + T(0.5) * dif.x, ys.y + T(0.5) * dif.y};
-            buf[ct_pad(N - m)] = V{ys.x - T(0.5) * dif.x, ys.y - T(0.5) * dif.y};
+            up[ct_off(it * TP)] = V{ys.x + T(0.5) * dif.x, ys.y + T(0.5) * dif.y};
+            dn[-ct_off(it * TP)] = V{ys.x - T(0.5) * dif.x, ys.y - T(0.5) * dif.y};
         }
     }
 }
@@ -332,20 +375,23 @@ __device__ __forceinline__ void dst_post(cplx_t<T>* buf, int tid, int gid, cplx_
     using V = cplx_t<T>;
     constexpr int half = N >> 1;
     constexpr int C = (half + TP - 1) / TP;
+    constexpr bool run = C > 1 && 8 % C == 0 && half == C * TP;   // a thread's k lie in one pad period
     const int k0 = tid * C;
+    const V* up = buf + ct_pad(k0);           // slots k0 + t
+    const V* dn = buf + ct_pad(N - k0 - C);   // slots N − k0 − t, t ≥ 1
     V D[C], O[C];
     V tot = V{T(0), T(0)};
 #pragma unroll
     for (int t = 0; t < C; ++t) {
         const int k = k0 + t;
-        if (k < half) {
-            const V zk = buf[ct_pad(k)];
+        if (run || k < half) {
+            const V zk = run ? up[t] : buf[ct_pad(k)];
             V d;
             if (k == 0) {
                 d = zk;
                 O[t] = V{T(0), T(0)};
             } else {
-                const V zn = buf[ct_pad(N - k)];
+                const V zn = run && t > 0 ? dn[C - t] : buf[ct_pad(N - k)];
                 d = cadd(zk, zn);
                 const V dl = csub(zk, zn);
                 O[t] = V{dl.y, -dl.x};  // −i (Z_k − Z_{N−k})
@@ -359,7 +405,7 @@ __device__ __forceinline__ void dst_post(cplx_t<T>* buf, int tid, int gid, cplx_
 #pragma unroll
     for (int t = 0; t < C; ++t) {
         const int k = k0 + t;
-        if (k < half) {
+        if (run || k < half) {
             emit(2 * k, cadd(ex, D[t]));
             if (k > 0) emit(2 * k - 1, O[t]);
         }
@@ -367,10 +413,10 @@ __device__ __forceinline__ void dst_post(cplx_t<T>* buf, int tid, int gid, cplx_
 }
 
 // One DST-I of a line pair: load → pre → FFT (plan PL) → post → emit.
-template <int N, int TP, int G, class T, int PL = 0, class Load, class Emit>
+template <int N, int TP, int G, class T, int PL = 0, class Load, class Fix, class Emit>
 __device__ __forceinline__ void dst_pair(cplx_t<T>* buf, const cplx_t<T>* W, const T* s, int tid, int gid,
-                                         Load load, Emit emit) {
-    dst_pre<N, TP, T>(buf, s, tid, load);
+                                         Load load, Fix fix, Emit emit) {
+    dst_pre<N, TP, T>(buf, s, tid, load, fix);
     gsync<TP, G>(gid);
     fft_stages<N, TP, G, 0, 1, T, PL>(buf, W, tid, gid);
     dst_post<N, TP, G, T>(buf, tid, gid, buf + ct_pad(N), emit);
@@ -443,11 +489,14 @@ __global__ void __launch_bounds__(ct_groups(N, PL) * ct_tp(N, PL), ct_fine(N, PL
     const int gid = threadIdx.x / TP, tid = threadIdx.x % TP;
     V* buf = bufs + gid * ct_buf(N);
     constexpr bool RES = x_res<LOAD>();
-    const int la = a.line0 + 2 * (blockIdx.x * G + gid);
-    if (la >= a.line1) return;  // the whole group leaves together
-    const bool hasb = (la + 1) < a.line1;
-    const int y = blockIdx.y;
     const int P = g.P, n1 = g.n1, n2 = g.n2;
+    // the group's line pairs: with ct_loop a 1-D grid of resident CTAs walks
+    // over all pairs of all slabs, else each group takes one pair (2-D grid)
+    const int pairs = (a.line1 - a.line0 + 1) / 2, items = pairs * (ct_loop(N) ? a.nslabs : 1);
+    for (int item = blockIdx.x * G + gid; item < items; item += gridDim.x * G) {
+    const int y = ct_loop(N) ? item / pairs : (int)blockIdx.y;
+    const int la = a.line0 + 2 * (ct_loop(N) ? item - y * pairs : item);
+    const bool hasb = (la + 1) < a.line1;
     const long long ioff = a.in_map.off(y) + (long long)la * P;
 
     CoarseBC cb;
@@ -501,13 +550,6 @@ __global__ void __launch_bounds__(ct_groups(N, PL) * ct_tp(N, PL), ct_fine(N, PL
         nb += c[N];
         return 4.0 * c[0] - nb;
     };
-    auto line_val = [&](const double* row, int i, int j) -> double {
-        double v = row[i];
-        if constexpr (LOAD == XLOAD_BC) {
-            if (cb.rc) v = with_bc(v, i, j);
-        }
-        return v;
-    };
     auto res_val = [&](int i, int r) -> double {
         double v = rs[(4 + r) * N + i];
         if constexpr (LOAD == XLOAD_RES_LAP) {
@@ -518,22 +560,32 @@ __global__ void __launch_bounds__(ct_groups(N, PL) * ct_tp(N, PL), ct_fine(N, PL
         }
         return v;
     };
+    // A pair without its second line loads the first one twice; the second
+    // line's result is not stored.
+    const int Pb = hasb ? P : 0;
     auto load = [&](int i) -> V {
         if constexpr (LOAD == XLOAD_F32) {
             const float* ra = static_cast<const float*>(a.in) + ioff;
-            return V{ra[i], hasb ? ra[i + P] : 0.0f};
+            return V{ra[i], ra[i + Pb]};
         } else if constexpr (LOAD == XLOAD_SUM || LOAD == XLOAD_F32_SUM) {
             const T* ra = static_cast<const T*>(a.in) + ioff;
             const T* rb = static_cast<const T*>(a.in2) + a.in2_map.off(y) + (long long)la * P;
-            return V{ra[i] + rb[i], hasb ? ra[i + P] + rb[i + P] : T(0)};
+            return V{ra[i] + rb[i], ra[i + Pb] + rb[i + Pb]};
         } else if constexpr (RES) {
             return V{(T)res_val(i, 0), hasb ? (T)res_val(i, 1) : T(0)};
         } else {
             const double* ra = static_cast<const double*>(a.in) + ioff;
-            const double va = line_val(ra, i, la);
-            const double vb = hasb ? line_val(ra + P, i, la + 1) : 0.0;
-            return V{(T)va, (T)vb};
+            return V{(T)ra[i], (T)ra[i + Pb]};
         }
+    };
+    auto fix = [&](int i, V v) -> V {
+        if constexpr (LOAD == XLOAD_BC) {
+            if (cb.rc) {
+                v.x = with_bc(v.x, i, la);
+                if (hasb) v.y = with_bc(v.y, i, la + 1);
+            }
+        }
+        return v;
     };
     // Stores that read what they update: fetch those values before the
     // transform, so their latency overlaps it (each thread owns the same
@@ -549,26 +601,24 @@ __global__ void __launch_bounds__(ct_groups(N, PL) * ct_tp(N, PL), ct_fine(N, PL
         const double* xa = READ_AUX ? a.aux + a.aux_map.off(y) + (long long)la * P : nullptr;
 #pragma unroll
         for (int k = 0; k < EO; ++k) {
-            const int o = tid + k * TP;
-            if (o < n1) {
-                if constexpr (READ_OUT) {
-                    po[k][0] = oa[o];
-                    po[k][1] = hasb ? oa[o + P] : 0.0;
-                }
-                if constexpr (READ_AUX) {
-                    px[k][0] = xa[o];
-                    px[k][1] = hasb ? xa[o + P] : 0.0;
-                }
+            const int o = min(tid + k * TP, n1 - 1);
+            if constexpr (READ_OUT) {
+                po[k][0] = oa[o];
+                po[k][1] = oa[o + Pb];
+            }
+            if constexpr (READ_AUX) {
+                px[k][0] = xa[o];
+                px[k][1] = xa[o + Pb];
             }
         }
     }
-    dst_pair<N, TP, G, T, PL>(buf, tw, sn, tid, gid, load, [&](int o, V v) { buf[ct_pad(o)] = v; });
+    dst_pair<N, TP, G, T, PL>(buf, tw, sn, tid, gid, load, fix, [&](int o, V v) { buf[ct_pad(o)] = v; });
     gsync<TP, G>(gid);
 #pragma unroll
     for (int k = 0; k < EO; ++k) {
         const int o = tid + k * TP;
         if (o >= n1) break;
-        const V v = buf[ct_pad(o)];
+        const V v = buf[ct_pad(tid) + ct_off(k * TP)];
         if constexpr (EMIT == XEMIT_F32) {
             float* oa = static_cast<float*>(a.out) + ooff;
             oa[o] = (float)v.x;
@@ -607,6 +657,9 @@ __global__ void __launch_bounds__(ct_groups(N, PL) * ct_tp(N, PL), ct_fine(N, PL
                 }
             }
         }
+    }
+    if constexpr (!ct_loop(N)) break;
+    gsync<TP, G>(gid);   // the next pair's transform writes the buffer read above
     }
 }
 
@@ -699,6 +752,7 @@ __global__ void __launch_bounds__(ct_tp(N, PL)) dst_lines_kernel(const T* Y, Sla
         double* rowT = smp + nx / 2 + 1;
         dst_pair<N, TP, 1, double, PL>(buf, tw, sn, threadIdx.x, 0,
                                        [&](int i) -> V { return V{(double)ra[i], (double)rb[i]}; },
+                                       [](int, V v) { return v; },
                                        [&](int o, V v) {
                                            if (o >= o0 && o <= o1) {
                                                rowB[o - o0] = v.x;
@@ -744,8 +798,18 @@ cudaError_t launch_x_n(const Geom& g, const DstPlan& px, const XPassArgs& a, cud
     const int lines = a.line1 - a.line0;
     if (lines <= 0 || a.nslabs <= 0) return cudaSuccess;
     const int pairs = (lines + 1) / 2;
-    dim3 grid((pairs + G - 1) / G, a.nslabs);
     const size_t smem = x_smem_bytes<N, LOAD, PL>();
+    dim3 grid((pairs + G - 1) / G, a.nslabs);
+    if constexpr (ct_loop(N)) {
+        static const int resident = [smem] {
+            int dev = 0, sms = 0, per = 0;
+            cudaGetDevice(&dev);
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, dst_x_kernel<N, LOAD, EMIT, PL>, G * TP, smem);
+            return std::max(1, sms * per);
+        }();
+        grid = dim3(std::min((pairs * a.nslabs + G - 1) / G, resident), 1);
+    }
     return launch_k(dst_x_kernel<N, LOAD, EMIT, PL>, grid, dim3(G * TP), smem, st, a, g, px);
 }
 

@@ -197,14 +197,11 @@ __global__ void __launch_bounds__(TX * LPM * E, ys_min_blocks<C, TX * LPM * E>()
         double RE = R;                                   // R^E
 #pragma unroll
         for (int s = 1; s < E; s <<= 1) RE *= RE;
-        const int L = nc / E, lb = l < L ? L - 1 - l : 0;   // lanes in use (E divides nc), distance to the last
-        double pw = RE, Rl = 1.0, Rb = 1.0;              // → R^{lE}, R^{(L−1−l)E}
+        double pw = RE;
 #pragma unroll
         for (int off = 1; off < LPM; off <<= 1) {
             const double n = __shfl_up_sync(0xffffffffu, inc, off, LPM);
             if (l >= off) inc = fma(pw, n, inc);
-            if (l & off) Rl *= pw;
-            if (lb & off) Rb *= pw;
             pw *= pw;
         }
         double run = __shfl_up_sync(0xffffffffu, inc, 1, LPM);
@@ -229,24 +226,36 @@ __global__ void __launch_bounds__(TX * LPM * E, ys_min_blocks<C, TX * LPM * E>()
         const double h0 = __shfl_sync(0xffffffffu, inc, 0, LPM) * sC[2 * TX + sm];   // w_0 / (1 − R^{2nc})
         run = __shfl_down_sync(0xffffffffu, inc, 1, LPM);
         if (l == LPM - 1) run = 0.0;
+#pragma unroll
+        for (int e = E - 1; e >= 0; --e) {               // B[e] ← first w of the next chunk
+            const double own_w = B[e];
+            B[e] = run;
+            run = fma(R, run, own_w);
+        }
+        const int L = nc / E, lb = l < L ? L - 1 - l : 0;   // lanes in use (E divides nc), distance to the last
+        double Rl = 1.0, Rb = 1.0;                       // → R^{lE}, R^{(L−1−l)E}
+        pw = RE;
+#pragma unroll
+        for (int off = 1; off < LPM; off <<= 1) {
+            if (l & off) Rl *= pw;
+            if (lb & off) Rb *= pw;
+            pw *= pw;
+        }
         double Rn = __shfl_sync(0xffffffffu, Rb, 0, LPM);   // R^{(L−1)E} → R^{nc}
 #pragma unroll
         for (int e = 0; e < E; ++e) Rn *= R;
-        double dn = Rn * Rb;                             // R^{2nc−c−1} of the lane's last chunk c = lE + E − 1
-        double up[E];                                    // R^{lE + e}
-        up[0] = Rl;
-#pragma unroll
-        for (int e = 1; e < E; ++e) up[e] = up[e - 1] * R;
         const double g0 = -h0 * sC[3 * TX + sm];
 #pragma unroll
-        for (int e = E - 1; e >= 0; --e) {
+        for (int e = 0; e < E; ++e) {
             const int cc = l * E + e;
+            double dn = Rn * Rb;                         // R^{2nc−cc−1}: from the lane's last chunk down
+#pragma unroll
+            for (int u = e; u < E - 1; ++u) dn *= R;
             if (cc < nc) {
-                sW[sm * LC + cc] = fma(-h0, up[e] * R - dn, run);   // first w of chunk cc+1
-                sV[sm * LC + cc] = fma(g0, up[e], A[e]);            // carry into chunk cc
+                sW[sm * LC + cc] = fma(-h0, Rl * R - dn, B[e]);   // first w of chunk cc+1
+                sV[sm * LC + cc] = fma(g0, Rl, A[e]);             // carry into chunk cc
             }
-            run = fma(R, run, B[e]);
-            dn *= R;
+            Rl *= R;
         }
     }
     __syncthreads();
