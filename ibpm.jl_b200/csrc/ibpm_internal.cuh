@@ -465,6 +465,20 @@ cudaError_t launch_stress_src(const BodyDev& b, const double* Fb, double h, doub
 cudaError_t launch_unit_src(const Geom& g, const BodyDev& b, int col0, int ncol, double* G,
                             long long bstride, cudaStream_t st);
 
+// Transfers from and to page-locked host memory by a kernel (hostio.cu): every
+// piece of a state in one launch, and a call's force history with the status word.
+struct PackPiece {
+    double* dev;
+    double* host;            // page-locked, contiguous
+    long long n;             // values
+    int n1, P;               // rows of n1 values, P apart on the device (n1 = P: contiguous)
+};
+struct PackArgs { PackPiece piece[6]; };
+constexpr size_t kPackBytes = (size_t)4 << 20;
+cudaError_t launch_pack(const PackArgs& a, int npieces, bool to_device, cudaStream_t st);
+cudaError_t launch_readback(const double* hist, double* out, int n, const int* status, int* status_out,
+                            cudaStream_t st);
+
 // Dense linear algebra (linalg.cu): in-place inverse by Gauss–Jordan with
 // partial pivoting of the row-major n×n matrix A; `work` holds
 // gj_work_doubles(n) doubles and `info` one int (set to the failing column + 1
