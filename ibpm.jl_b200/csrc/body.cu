@@ -374,34 +374,6 @@ cudaError_t launch_stress_src(const BodyDev& b, const double* Fb, double h, doub
                     Gsrc);
 }
 
-// C'E' e_kk for unit forces kk = col0 + r (B_times!, laplacian.jl:162), written
-// into the level-1 slab of batch member r (slab zeroed beforehand).  One thread
-// per point of the 14×14 box of Γ points the 13×13 flux window can reach.
-__global__ void unit_src_kernel(BodyDev b, Geom g, int col0, int ncol, double* G, long long bstride) {
-    pdl_wait();
-    pdl_trigger();
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= ncol * 196) return;
-    const int r = t / 196, ab = t % 196, da = ab / 14, db = ab % 14;
-    const int kk = col0 + r;
-    const int comp = kk / b.nb, k = kk % b.nb;
-    const int bx = b.bidx[k], by = b.bidx[b.nb + k];
-    const double* w = b.w + (long long)kk * 169;
-    const int gi = bx - 7 + da, gj = by - 7 + db;  // Julia Γ index
-    if (gi < 1 || gi > g.n1 || gj < 1 || gj > g.n2) return;
-    auto qx = [&](int I, int J) -> double {
-        const int l = I - bx + 6, m = J - by + 6;
-        return (comp == 0 && l >= 0 && l < 13 && m >= 0 && m < 13) ? w[l * 13 + m] : 0.0;
-    };
-    auto qy = [&](int I, int J) -> double {
-        const int l = I - bx + 6, m = J - by + 6;
-        return (comp == 1 && l >= 0 && l < 13 && m >= 0 && m < 13) ? w[l * 13 + m] : 0.0;
-    };
-    // Γ[i-1, j-1] = (qx[i, j-1] − qx[i, j]) + (qy[i, j] − qy[i-1, j]), (i, j) = (gi+1, gj+1)
-    const double v = (qx(gi + 1, gj) - qx(gi + 1, gj + 1)) + (qy(gi + 1, gj + 1) - qy(gi, gj + 1));
-    G[(long long)r * bstride + (long long)(gj - 1) * g.P + (gi - 1)] = v;
-}
-
 // ---------------------------------------------------------------------------
 // Bodies moved by a MotionFunction (move_body!, move-body-utils.jl:86-133):
 // point p of body j at the step's row r = (x, y, cos θ, sin θ, ẋ, ẏ, θ̇) of the
@@ -498,13 +470,6 @@ __global__ void info_to_status_kernel(const int* info, int* status) {
 
 cudaError_t launch_info_to_status(const int* info, int* status, cudaStream_t st) {
     info_to_status_kernel<<<1, 1, 0, st>>>(info, status);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_unit_src(const Geom& g, const BodyDev& b, int col0, int ncol, double* G, long long bstride,
-                            cudaStream_t st) {
-    const int n = ncol * 196;
-    unit_src_kernel<<<(n + 255) / 256, 256, 0, st>>>(b, g, col0, ncol, G, bstride);
     return cudaGetLastError();
 }
 

@@ -168,6 +168,14 @@ __global__ void bt_unit_src_kernel(Geom g, int c0, int ncol, double* G, long lon
     G[(long long)b * bstride + (long long)j * g.P + i] = 1.0;
 }
 
+// get_bc! in the edge order bottom, top, left, right.
+__device__ __forceinline__ double edge_entry(const Geom& g, const CoarseBC& cb, int m) {
+    if (m < g.n1) return cb.bot(m + 1);
+    if (m < 2 * g.n1) return cb.top(m - g.n1 + 1);
+    if (m < 2 * g.n1 + g.n2) return cb.left(m - 2 * g.n1 + 1);
+    return cb.right(m - 2 * g.n1 - g.n2 + 1);
+}
+
 // R[m, c0 + b] = get_bc! entry m of the solve in slab b.
 __global__ void bt_gather_kernel(Geom g, int c0, int ncol, const double* psi, long long bstride, double* R) {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
@@ -176,12 +184,19 @@ __global__ void bt_gather_kernel(Geom g, int c0, int ncol, const double* psi, lo
     if (m >= nE || b >= ncol) return;
     CoarseBC cb;
     cb.rc = psi + (long long)b * bstride; cb.P = g.P; cb.nx = g.nx; cb.ny = g.ny;
-    double v;
-    if (m < g.n1) v = cb.bot(m + 1);
-    else if (m < 2 * g.n1) v = cb.top(m - g.n1 + 1);
-    else if (m < 2 * g.n1 + g.n2) v = cb.left(m - 2 * g.n1 + 1);
-    else v = cb.right(m - 2 * g.n1 - g.n2 + 1);
-    R[(long long)m * ep + c0 + b] = v;
+    R[(long long)m * ep + c0 + b] = edge_entry(g, cb, m);
+}
+
+// Bottom entries at 0, top at nx, left at 2 nx, right at 2 nx + ny.
+__global__ void edges_of_psi_kernel(Geom g, const double* psi, long long bstride, double* e) {
+    pdl_wait();
+    pdl_trigger();
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= 2 * g.n1 + 2 * g.n2) return;
+    CoarseBC cb;
+    cb.rc = psi + (long long)blockIdx.y * bstride; cb.P = g.P; cb.nx = g.nx; cb.ny = g.ny;
+    const int at = m < g.n1 ? m : m < 2 * g.n1 ? m + 1 : m < 2 * g.n1 + g.n2 ? m + 2 : m + 3;
+    e[(long long)blockIdx.y * (2 * g.nx + 2 * g.ny) + at] = edge_entry(g, cb, m);
 }
 
 // Run f(t0, t1) over [0, n) split across the host's threads.
@@ -356,6 +371,12 @@ cudaError_t launch_bt_expand(const Geom& g, const BtChainArgs& a, cudaStream_t s
 #undef IBPM_CASE
         default: return cudaErrorInvalidValue;
     }
+}
+
+cudaError_t launch_edges_of_psi(const Geom& g, const double* psi, long long bstride, int nbatch, double* e,
+                                cudaStream_t st) {
+    dim3 grid((bt_edge_len(g) + 127) / 128, nbatch);
+    return launch_k(edges_of_psi_kernel, grid, dim3(128), 0, st, g, psi, bstride, e);
 }
 
 cudaError_t launch_bt_unit_src(const Geom& g, int c0, int ncol, double* G, long long bstride, cudaStream_t st) {

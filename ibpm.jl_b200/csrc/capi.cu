@@ -100,7 +100,7 @@ struct ibpm_handle {
     double* d_ub = nullptr;                // body-point velocities (nb, 2)
     int* d_bbox = nullptr;                 // min/max body_idx of the step
     double* btab = nullptr; int btab_cap = 0;
-    double *bGB = nullptr, *bPB = nullptr, *bwork = nullptr;  // per-step B rebuild
+    double *bGB = nullptr, *bPB = nullptr, *bEB = nullptr, *bwork = nullptr;  // per-step B rebuild
     int* binfo = nullptr;
     // discrete adjoint (allocated by the first ibpm_adjoint_run)
     int adj_k = 0, adj_ncp = 0, adj_nsteps = 0;
@@ -764,6 +764,69 @@ static int enqueue_step_refined(ibpm_handle* h, int p, int nsw) {
     return h->bt ? vort2flux_refined_bt(h, Gnew, nsw, h->q, mg, mg) : vort2flux_refined(h, Gnew, nsw, h->q, mg);
 }
 
+// Columns [c0, c0 + R) of B, B[:, j] = E · vort2flux(A⁻¹₁ C'E' e_j)[level-1 flux]
+// (B_times!, laplacian.jl:143-169), into h->Binv.  GB and PB hold mg slabs per
+// column, EB the edge values of one level; GB is zero outside what this writes (the centres of
+// the coarser levels).  A column's vort2flux! needs less than a state's:
+//   * the x-spectrum of C'E' e_j and A⁻¹'s y-solve are one launch from the 196
+//     values of the source, and the level-1 Δ⁻¹ starts from that spectrum;
+//   * Γ of a coarser level is zero outside its centre: only those rows are
+//     transformed, of all levels at once;
+//   * the edge values of the next coarser ψ (curl.jl:151-158) enter in the
+//     y-solve (YSRC_BOTH), and ψ of a coarser level is needed only between its
+//     sample lines, ψ of level 1 only around the bodies.
+// What bounds it: the transforms of R·mg slabs.  With memset, source, full
+// forward and inverse passes on every level the 102 columns of 400x200 x 5 took
+// 1290 µs per step, this way 720.
+static int unit_columns(ibpm_handle* h, int c0, int R, double* GB, double* PB, double* EB, bool moving) {
+    const Geom& g = h->g;
+    const int mg = g.mg;
+    const long long bs = g.S * mg;
+    const double slab = 8.0 * g.n1 * g.n2 * R;
+    const int* box = moving ? h->d_bbox : nullptr;
+    YSource ys;
+    ys.edges.sx = h->px.s; ys.edges.nx = g.nx;
+    ys.bidx = h->body.bidx; ys.w = h->body.w; ys.nb = h->nb; ys.col0 = c0;
+    SlabMap l0 = levmap(g, 0, 1, bs);
+    LAUNCH(K_DSTY, slab, launch_y_solve_unit(g, PB, l0, R, spec(h, SPEC_AINV), ys, h->st));
+    auto xpass = [&](const double* in, double* out, SlabMap m, int nslabs, int y0, int y1, const int* rowbox) {
+        XPassArgs a{};
+        a.in = in; a.out = out; a.in_map = m; a.out_map = m; a.nslabs = nslabs; a.line0 = y0; a.line1 = y1;
+        a.load = XLOAD_PLAIN; a.emit = XEMIT_STORE; a.rowbox = rowbox;
+        return launch_dst_x(g, h->px, a, h->st);
+    };
+    const int s0 = g.ny / 4 - 1, s1 = 3 * g.ny / 4;      // rows between the sample lines, [s0, s1)
+    if (mg > 1) {
+        LAUNCH(K_DSTX, 2 * slab, xpass(PB, GB, l0, R, 0, g.n2, nullptr));
+        for (int lev = 1; lev < mg; ++lev)
+            LAUNCH(K_COARSIFY, 1.25 * slab,
+                   launch_coarsify(g, GB, levmap(g, lev - 1, 1, bs), levmap(g, lev, 1, bs), R, h->st));
+        LAUNCH(K_DSTX, (mg - 1) * slab, xpass(GB, PB, levmap(g, 1, mg - 1, bs), (mg - 1) * R, s0 + 1, s1 - 1, nullptr));
+    }
+    for (int lev = mg - 1; lev >= 0; --lev) {
+        SlabMap m = levmap(g, lev, 1, bs);
+        ys.hat = lev < mg - 1 ? EB : nullptr;
+        if (ys.hat) {
+            // the bottom and top entries as one line pair per column (inside the
+            // y-solve their sums cost 80 µs of its 114 over 102 columns)
+            LAUNCH(K_BTCHAIN, 16.0 * bt_edge_len(g) * R, launch_edges_of_psi(g, PB + (lev + 1) * g.S, bs, R, EB, h->st));
+            SlabMap em{1, 0, 2ll * g.nx + 2 * g.ny, 0};
+            LAUNCH(K_DSTX, 32.0 * g.n1 * R, xpass(EB, EB, em, R, 0, 2, nullptr));
+        }
+        const bool fine = lev == 0;
+        ys.in_scale = fine ? 2.0 * g.nx : 1.0;           // level 1: from the solved spectrum, scaled by 1/(2 nx)
+        ys.in0 = fine ? 0 : s0 + 1; ys.in1 = fine ? g.n2 : s1 - 1;
+        ys.out0 = fine ? h->win_y0 : s0; ys.out1 = fine ? h->win_y1 : s1;
+        ys.rowbox = fine ? box : nullptr;
+        LAUNCH(K_DSTY, 1.5 * slab, launch_y_solve_both(g, PB, m, R, spec(h, SPEC_DELTA), ys, h->st));
+        LAUNCH(K_DSTX, 2 * slab * (ys.out1 - ys.out0) / g.n2,
+               xpass(PB, PB, m, R, box && fine ? 0 : ys.out0, box && fine ? g.n2 : ys.out1, ys.rowbox));
+    }
+    LAUNCH(K_E, 16.0 * 169 * R,
+           launch_E(g, h->body, PB, bs, R, 0.0, 0.0, h->Binv + c0, -(long long)h->nf, false, h->st));
+    return IBPM_OK;
+}
+
 // update_bodies! for MotionFunction bodies (timestepping.jl:386-398): move the
 // points to this step's row of the motion table, recompute body_idx and the
 // weights of E, and rebuild B⁻¹ from B_times! (laplacian.jl:143-169) by the
@@ -778,17 +841,9 @@ static int enqueue_body_update(ibpm_handle* h) {
                              h->d_ub, h->d_bbox, h->status, h->st));
     LAUNCH(K_E, 8.0 * 169 * h->nf, launch_weights(g, h->h, h->offx, h->offy, h->body, h->st));
     const int chunk = std::min(nf, kBChunk);
-    const long long bstride = g.S * g.mg;
     for (int c0 = 0; c0 < nf; c0 += chunk) {
-        const int R = std::min(chunk, nf - c0);
-        CK(cudaMemsetAsync(h->bGB, 0, sizeof(double) * bstride * R, h->st));
-        LAUNCH(K_SRC, 8.0 * 196 * R, launch_unit_src(g, h->body, c0, R, h->bGB, bstride, h->st));
-        SlabMap l0 = levmap(g, 0, 1, bstride);
-        int rc = poisson(h, h->bGB, l0, h->bGB, l0, h->bGB, l0, R, SPEC_AINV, XEMIT_STORE);
+        int rc = unit_columns(h, c0, std::min(chunk, nf - c0), h->bGB, h->bPB, h->bEB, true);
         if (rc) return rc;
-        rc = vort2flux(h, h->bGB, h->bPB, bstride, R, nullptr, 0, 0);
-        if (rc) return rc;
-        LAUNCH(K_E, 16.0 * 169 * R, launch_E(g, h->body, h->bPB, bstride, R, 0.0, 0.0, h->Binv + c0, -(long long)nf, false, h->st));
     }
     LAUNCH(K_GEMV, 8.0 * 4.0 * nf * nf, launch_gj_inverse(h->Binv, nf, h->bwork, h->binfo, h->st));
     LAUNCH(K_GEMV, 8.0, launch_info_to_status(h->binfo, h->status, h->st));
@@ -908,14 +963,14 @@ static int build_binv(ibpm_handle* h) {
     const Geom& g = h->g;
     const int nf = h->nf, mg = g.mg;
     const int chunk = std::min(nf, kBChunk);
-    double *GB = nullptr, *PB = nullptr, *work = nullptr;
+    double *GB = nullptr, *PB = nullptr, *EB = nullptr, *work = nullptr;
     int* info = nullptr;
     int rc;
     const long long bstride = g.S * mg;
     if ((rc = dalloc(h, &GB, (size_t)bstride * chunk)) || (rc = dalloc(h, &PB, (size_t)bstride * chunk)) ||
-        (rc = dalloc(h, &work, gj_work_doubles(nf))) ||
+        (rc = dalloc(h, &EB, (size_t)(2 * g.nx + 2 * g.ny) * chunk)) || (rc = dalloc(h, &work, gj_work_doubles(nf))) ||
         (rc = dalloc(h, &info, 1))) {
-        cudaFree(GB); cudaFree(PB); cudaFree(work); cudaFree(info);
+        cudaFree(GB); cudaFree(PB); cudaFree(EB); cudaFree(work); cudaFree(info);
         return rc;
     }
     // B at create is built with the single-level (latency) plan on every
@@ -925,22 +980,11 @@ static int build_binv(ibpm_handle* h) {
     h->px.planN = h->px.plan1;
     auto cleanup = [&]() {
         h->px.planN = planN;
-        cudaFree(GB); cudaFree(PB); cudaFree(work); cudaFree(info);
+        cudaFree(GB); cudaFree(PB); cudaFree(EB); cudaFree(work); cudaFree(info);
     };
-    for (int c0 = 0; c0 < nf && rc == IBPM_OK; c0 += chunk) {
-        const int R = std::min(chunk, nf - c0);
-        if (cudaMemsetAsync(GB, 0, sizeof(double) * bstride * R, h->st) != cudaSuccess) { rc = IBPM_ERR_CUDA; break; }
-        if (launch_unit_src(g, h->body, c0, R, GB, bstride, h->st) != cudaSuccess) { rc = IBPM_ERR_CUDA; break; }
-        SlabMap l0 = levmap(g, 0, 1, bstride);
-        rc = poisson(h, GB, l0, GB, l0, GB, l0, R, SPEC_AINV, XEMIT_STORE);
-        if (rc) break;
-        rc = vort2flux(h, GB, PB, bstride, R, nullptr, 0, 0);  // ψ of each column
-        if (rc) break;
-        if (launch_E(g, h->body, PB, bstride, R, 0.0, 0.0, h->Binv + c0, -(long long)nf, false, h->st) != cudaSuccess) {
-            rc = IBPM_ERR_CUDA;
-            break;
-        }
-    }
+    if (cudaMemsetAsync(GB, 0, sizeof(double) * bstride * chunk, h->st) != cudaSuccess) rc = fail(h, IBPM_ERR_CUDA, "B setup: memset");
+    for (int c0 = 0; c0 < nf && rc == IBPM_OK; c0 += chunk)
+        rc = unit_columns(h, c0, std::min(chunk, nf - c0), GB, PB, EB, false);
     if (rc == IBPM_OK) {
         if (launch_gj_inverse(h->Binv, nf, work, info, h->st) != cudaSuccess) rc = fail(h, IBPM_ERR_CUDA, "gj inverse launch");
     }
@@ -969,7 +1013,7 @@ static void free_handle(ibpm_handle* h) {
         if (p) cudaFree(p);
     if (h->mtab) cudaFree(h->mtab);
     for (void* p : {(void*)h->d_x0, (void*)h->d_ub, (void*)h->d_bbox, (void*)h->btab, (void*)h->bGB, (void*)h->bPB,
-                    (void*)h->bwork, (void*)h->binfo})
+                    (void*)h->bEB, (void*)h->bwork, (void*)h->binfo})
         if (p) cudaFree(p);
     if (h->GB) cudaFree(h->GB);
     if (h->qB) cudaFree(h->qB);
@@ -1457,8 +1501,10 @@ extern "C" int ibpm_set_motion_function(ibpm_handle* h) {
     if ((rc = dalloc(h, &h->d_x0, 2 * h->nb)) || (rc = dalloc(h, &h->d_ub, 2 * h->nb)) ||
         (rc = dalloc(h, &h->d_bbox, 4)) || (rc = dalloc(h, &h->bGB, (size_t)bstride * chunk)) ||
         (rc = dalloc(h, &h->bPB, (size_t)bstride * chunk)) ||
+        (rc = dalloc(h, &h->bEB, (size_t)(2 * g.nx + 2 * g.ny) * chunk)) ||
         (rc = dalloc(h, &h->bwork, gj_work_doubles(nf))) || (rc = dalloc(h, &h->binfo, 1)))
         return rc;
+    CK(cudaMemsetAsync(h->bGB, 0, sizeof(double) * bstride * chunk, h->st));   // unit_columns writes the centres only
     // the reference configuration x0 is the body as created (RigidBody.x0)
     CK(cudaMemcpyAsync(h->d_x0, h->d_xb, sizeof(double) * 2 * h->nb, cudaMemcpyDeviceToDevice, h->st));
     CK(cudaMemsetAsync(h->d_ub, 0, sizeof(double) * 2 * h->nb, h->st));

@@ -492,11 +492,13 @@ __global__ void __launch_bounds__(ct_groups(N, PL) * ct_tp(N, PL), ct_fine(N, PL
     const int P = g.P, n1 = g.n1, n2 = g.n2;
     // the group's line pairs: with ct_loop a 1-D grid of resident CTAs walks
     // over all pairs of all slabs, else each group takes one pair (2-D grid)
-    const int pairs = (a.line1 - a.line0 + 1) / 2, items = pairs * (ct_loop(N) ? a.nslabs : 1);
+    const int line0 = a.rowbox ? max(a.line0, a.rowbox[1] - kBoxBelow) : a.line0;
+    const int line1 = a.rowbox ? min(a.line1, a.rowbox[3] + kBoxAbove) : a.line1;
+    const int pairs = max(line1 - line0 + 1, 0) / 2, items = pairs * (ct_loop(N) ? a.nslabs : 1);
     for (int item = blockIdx.x * G + gid; item < items; item += gridDim.x * G) {
     const int y = ct_loop(N) ? item / pairs : (int)blockIdx.y;
-    const int la = a.line0 + 2 * (ct_loop(N) ? item - y * pairs : item);
-    const bool hasb = (la + 1) < a.line1;
+    const int la = line0 + 2 * (ct_loop(N) ? item - y * pairs : item);
+    const bool hasb = (la + 1) < line1;
     const long long ioff = a.in_map.off(y) + (long long)la * P;
 
     CoarseBC cb;

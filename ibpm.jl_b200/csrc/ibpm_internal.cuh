@@ -279,6 +279,7 @@ struct XPassArgs {
     const double* mcA;                           // per simulation of a batch group (in_map's batch), or nullptr
     int nslabs, line0, line1;
     int load, emit;
+    const int* rowbox;                           // moving bodies: only the lines E reads (YSource), or nullptr
 };
 cudaError_t launch_dst_x(const Geom& g, const DstPlan& px, const XPassArgs& a, cudaStream_t st);
 
@@ -315,6 +316,31 @@ struct BtSynth {
 // The y-solve of the edge vectors' x-spectrum into the slabs of `out`.
 cudaError_t launch_y_solve_edges(const Geom& g, void* out, SlabMap map, int nslabs, const SpecParams& sp,
                                  const BtSynth& bs, cudaStream_t st);
+// Other right-hand sides of a y-solve (ysolve.cu), FP64: part of the slab's rows
+// plus edge vectors, and unit forces.  rowbox is the device's min/max body_idx
+// (x, y, x, y) of moving bodies: E reads ψ of slab rows rowbox[1] − kBoxBelow …
+// rowbox[3] + kBoxAbove − 1.
+constexpr int kBoxBelow = 8, kBoxAbove = 6;
+enum YSrcKind { YSRC_DATA = 0, YSRC_EDGES = 1, YSRC_BOTH = 2, YSRC_UNIT = 3 };
+struct YSource {
+    BtSynth edges{nullptr, nullptr, 0};     // EDGES: e per batch member and level; sx, nx
+    const double* hat = nullptr;            // BOTH: per batch member (2 nx + 2 ny apart) the x-transforms of the
+                                            // bottom and top entries, nx apart, then left and right, ny apart
+    double in_scale = 1.0;                  // BOTH: factor on the slab's rows [in0, in1)
+    int in0 = 0, in1 = 0, out0 = 0, out1 = 0;
+    const int* rowbox = nullptr;            // BOTH: the rows stored instead of [out0, out1)
+    const int* bidx = nullptr;              // UNIT: points' body_idx, weights, point count
+    const double* w = nullptr;
+    int nb = 0, col0 = 0;
+};
+cudaError_t launch_y_solve_both(const Geom& g, double* data, SlabMap map, int nslabs, const SpecParams& sp,
+                                const YSource& ys, cudaStream_t st);
+cudaError_t launch_y_solve_unit(const Geom& g, double* data, SlabMap map, int nslabs, const SpecParams& sp,
+                                const YSource& ys, cudaStream_t st);
+// The entries that apply_bc! adds, get_bc! of the slabs ψ (bstride apart) of
+// nbatch fields, in the layout of YSource::hat (bottom and top not transformed).
+cudaError_t launch_edges_of_psi(const Geom& g, const double* psi, long long bstride, int nbatch, double* e,
+                                cudaStream_t st);
 // The line samples (FP64) of the levels of `map` from Y (FP32 when f32).
 cudaError_t launch_dst_lines(const Geom& g, const DstPlan& px, const void* Y, SlabMap map, int nslabs,
                              void* samples, int f32, cudaStream_t st);
@@ -462,9 +488,6 @@ cudaError_t launch_stress(const BodyDev& b, const double* Fb, double h, double d
 // launch_stress and the projection source C'E'F̃b in one launch (fixed bodies)
 cudaError_t launch_stress_src(const BodyDev& b, const double* Fb, double h, double dt, double* hist, int hist_cap,
                               int* counter, int* status, double* Gsrc, cudaStream_t st);
-cudaError_t launch_unit_src(const Geom& g, const BodyDev& b, int col0, int ncol, double* G,
-                            long long bstride, cudaStream_t st);
-
 // Transfers from and to page-locked host memory by a kernel (hostio.cu): every
 // piece of a state in one launch, and a call's force history with the status word.
 struct PackPiece {

@@ -49,25 +49,32 @@ __device__ __forceinline__ double pow_int(double b, int e) {
 // row are whole 32-byte sectors.  The constants of a mode depend on the
 // problem only and are formed before the dependency wait.
 //
-// SYNTH: f is not read but built, the x-spectrum of apply_bc!(e) of the slab's
-// level (BtSynth): with S(i, k) = 2 sin(π i k / nx),
-//     f(k, j) = S(1, k) e_L(j) + S(nx−1, k) e_R(j)
-//             + [j = 1] Σ_i S(i, k) e_B(i) + [j = ny−1] Σ_i S(i, k) e_T(i),
-// and the result goes to `out` (same slab map).
+// SRC, how f is formed:
+//   YSRC_DATA    read from the slab, solved in place
+//   YSRC_EDGES   the x-spectrum of apply_bc!(e) of the slab's level (BtSynth),
+//                into `out` (same slab map): with S(i, k) = 2 sin(π i k / nx),
+//                f(k, j) = S(1, k) e_L(j) + S(nx−1, k) e_R(j)
+//                        + [j = 1] Σ_i S(i, k) e_B(i) + [j = ny−1] Σ_i S(i, k) e_T(i)
+//   YSRC_BOTH    in_scale × the slab's rows [in0, in1) plus, where hat is given,
+//                the edges with their bottom and top sums already formed; only
+//                rows [out0, out1) (or the bodies', rowbox) stored
+//   YSRC_UNIT    the x-spectrum of C'E' e_kk of force component col0 + batch
+//                (B_times!, laplacian.jl:162), 14×14 values around its point
 // Resident CTAs per SM the register budget is set for: 1024 threads of at most
 // 64 registers, or 768 of 80 where a thread holds 16 rows.
 template <int C, int THREADS> constexpr int ys_min_blocks() {
     return THREADS > 512 ? 1 : (C > 8 ? 768 : 1024) / THREADS;
 }
 
-template <class T, int C, int TX, int LPM, int E, bool SYNTH>
+template <class T, int C, int TX, int LPM, int E, int SRC>
 __global__ void __launch_bounds__(TX * LPM * E, ys_min_blocks<C, TX * LPM * E>())
-    y_solve_kernel(T* data, SlabMap map, Geom g, const __grid_constant__ SpecParams sp, T* out, BtSynth bs) {
+    y_solve_kernel(T* data, SlabMap map, Geom g, const __grid_constant__ SpecParams sp, T* out,
+                   const __grid_constant__ YSource ys) {
     constexpr int LC = LPM * E + 1;                      // chunk pitch of the exchange arrays (odd)
     __shared__ double sV[TX * LC], sW[TX * LC];
     __shared__ double sC[4 * TX];                        // r, κ·scale, 1/(1−r^{2ny}), 1−r² of each mode
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    double* sn = reinterpret_cast<double*>(smem_raw);    // SYNTH: sin(π t/nx), t < nx
+    double* sn = reinterpret_cast<double*>(smem_raw);    // edges, unit: sin(π t/nx), t < nx
     const int P = g.P, n1 = g.n1, nx = g.nx, nc = g.ny / C;
     const int tid = threadIdx.x, x = tid % TX, c = tid / TX;
     const bool own = c < nc;                             // the block is padded to whole warps
@@ -90,22 +97,54 @@ __global__ void __launch_bounds__(TX * LPM * E, ys_min_blocks<C, TX * LPM * E>()
         sC[2 * TX + tid] = 1.0 / (1.0 - pow_int(r * r, g.ny));
         sC[3 * TX + tid] = 1.0 - r * r;
     }
-    if constexpr (SYNTH) {
-        for (int t = tid; t < nx; t += blockDim.x) sn[t] = bs.sx[t];
-    }
+    if constexpr (SRC == YSRC_UNIT || SRC == YSRC_EDGES)
+        for (int t = tid; t < nx; t += blockDim.x) sn[t] = ys.edges.sx[t];
     pdl_wait();
     pdl_trigger();
 
     // lane l of mode sm in the scan over the chunks
     const int sm = tid / LPM, l = tid % LPM;
     const bool scans = sm < TX;                          // whole warps
+    auto sinpix = [&](int t) -> double { return t < nx ? sn[t] : -sn[t - nx]; };   // 0 ≤ t < 2 nx
     double v[C];
-    if constexpr (SYNTH) {
+    if constexpr (SRC == YSRC_DATA || SRC == YSRC_BOTH) {
+        const T* src = data + soff;
+        T raw[C];
+#pragma unroll
+        for (int i = 0; i < C; ++i) {
+            const int j = c * C + i - 1;                 // slab row
+            const bool in = SRC == YSRC_DATA ? j >= 0 : j >= ys.in0 && j < ys.in1;
+            raw[i] = (own && in && col < n1) ? src[o0 + i * P] : T(0);
+        }
+        __syncthreads();                                 // sC, sn, while the loads are in flight
+#pragma unroll
+        for (int i = 0; i < C; ++i) v[i] = SRC == YSRC_DATA ? (double)raw[i] : ys.in_scale * (double)raw[i];
+    } else {
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < C; ++i) v[i] = 0.0;
+    }
+    // S(1, k) of the mode; S(nx−1, k) = (−1)^{k+1} S(1, k)
+    auto side = [&](const double* eL, const double* eR, double s1) {
+        const double sr = col & 1 ? -1.0 : 1.0;          // k = col + 1
+#pragma unroll
+        for (int i = 0; i < C; ++i) {
+            const int j = c * C + i - 1;
+            if (own && j >= 0) v[i] = fma(s1, fma(sr, __ldg(&eR[j]), __ldg(&eL[j])), v[i]);
+        }
+    };
+    if constexpr (SRC == YSRC_BOTH) {
+        if (ys.hat) {
+            const double* e = ys.hat + (long long)bt * (2 * nx + 2 * g.ny);
+            side(e + 2 * nx, e + 2 * nx + g.ny, 2.0 * __ldg(&ys.edges.sx[min(col + 1, nx - 1)]));
+            if (c == 0) v[1] += e[col];
+            if (c == nc - 1) v[C - 1] += e[nx + col];
+        }
+    }
+    if constexpr (SRC == YSRC_EDGES) {
         const int ep = (2 * n1 + 2 * g.n2 + 3) & ~3;
-        const double* e = bs.e + ((long long)bt * g.mg + lev) * ep;
+        const double* e = ys.edges.e + ((long long)bt * g.mg + lev) * ep;
         const int k = col + 1, nx2 = 2 * nx;
-        __syncthreads();                                 // sn, sC
-        auto sinpix = [&](int t) -> double { return t < nx ? sn[t] : -sn[t - nx]; };
         // this thread's share of the sine sums of the bottom and top rows
         if (own) {
             double pb = 0.0, pt = 0.0;
@@ -122,14 +161,7 @@ __global__ void __launch_bounds__(TX * LPM * E, ys_min_blocks<C, TX * LPM * E>()
             sV[x * LC + c] = pb;
             sW[x * LC + c] = pt;
         }
-        const double sl = 2.0 * sinpix(k % nx2), sr = 2.0 * sinpix((k * (nx - 1)) % nx2);
-        const double* eL = e + 2 * n1;
-        const double* eR = eL + g.n2;
-#pragma unroll
-        for (int i = 0; i < C; ++i) {
-            const int j = c * C + i - 1;                 // slab row
-            v[i] = own && j >= 0 ? fma(sl, __ldg(&eL[j]), sr * __ldg(&eR[j])) : 0.0;
-        }
+        side(e + 2 * n1, e + 2 * n1 + g.n2, 2.0 * sinpix(k % nx2));
         __syncthreads();
         if (scans) {                                     // sums over the chunks
             double b = 0.0, tt = 0.0;
@@ -152,14 +184,41 @@ __global__ void __launch_bounds__(TX * LPM * E, ys_min_blocks<C, TX * LPM * E>()
         if (c == 0) v[1] += sV[x * LC];
         if (c == nc - 1) v[C - 1] += sW[x * LC];
         __syncthreads();
-    } else {
-        const T* src = data + soff;
-        T raw[C];
+    }
+    if constexpr (SRC == YSRC_UNIT) {
+        __shared__ double src[14][15];                   // [row][column] of the box
+        const int kk = ys.col0 + bt, comp = kk / ys.nb, pt = kk % ys.nb;
+        const int bx = ys.bidx[pt], by = ys.bidx[ys.nb + pt];
+        const double* wt = ys.w + (long long)kk * 169;
+        for (int t = tid; t < 196; t += blockDim.x) {
+            const int da = t % 14, db = t / 14;
+            // Γ[gi, gj] = (qx[gi+1, gj] − qx[gi+1, gj+1]) + (qy[gi+1, gj+1] − qy[gi, gj+1]) of the window's
+            // weights (rot!, curl.jl:22-34), gi = bx − 7 + da, gj = by − 7 + db
+            auto at = [&](int l2, int m2) -> double {
+                return l2 >= 0 && l2 < 13 && m2 >= 0 && m2 < 13 ? wt[l2 * 13 + m2] : 0.0;
+            };
+            double val;
+            if (comp == 0) val = at(da, db - 1) - at(da, db);
+            else val = at(da, db) - at(da - 1, db);
+            const int gi = bx - 7 + da, gj = by - 7 + db;
+            src[db][da] = gi >= 1 && gi <= n1 && gj >= 1 && gj <= g.n2 ? val : 0.0;
+        }
+        __syncthreads();
+        const int k = col + 1, nx2 = 2 * nx, j0 = by - 7;    // grid row of the box's first row
+        if (own && c * C + C > j0 && c * C < j0 + 14) {
+            int t = (int)(((long long)max(bx - 7, 0) * k) % nx2);
+            const int a0 = max(7 - bx, 0);               // gi = 0 or below: no values there
+            for (int da = a0; da < 14; ++da) {
+                const double sv = 2.0 * sinpix(t);
 #pragma unroll
-        for (int i = 0; i < C; ++i) raw[i] = (own && c * C + i > 0 && col < n1) ? src[o0 + i * P] : T(0);
-        __syncthreads();                                 // sC, while the loads are in flight
-#pragma unroll
-        for (int i = 0; i < C; ++i) v[i] = (double)raw[i];
+                for (int i = 0; i < C; ++i) {
+                    const int db = c * C + i - j0;
+                    if (db >= 0 && db < 14) v[i] = fma(sv, src[db][da], v[i]);
+                }
+                t += k;
+                if (t >= nx2) t -= nx2;
+            }
+        }
     }
 
     // local recursions: v with zero carry, and the chunk's first w
@@ -273,19 +332,26 @@ __global__ void __launch_bounds__(TX * LPM * E, ys_min_blocks<C, TX * LPM * E>()
         w = fma(r, w, v[i]);
         v[i] = kap * w;
     }
-    T* dst = (SYNTH ? out : data) + soff;
+    T* dst = (SRC == YSRC_EDGES ? out : data) + soff;
+    int out0 = 0, out1 = g.n2;
+    if constexpr (SRC == YSRC_BOTH) {
+        out0 = ys.rowbox ? max(0, ys.rowbox[1] - kBoxBelow) : ys.out0;
+        out1 = ys.rowbox ? min(g.n2, ys.rowbox[3] + kBoxAbove) : ys.out1;
+    }
 #pragma unroll
-    for (int i = 0; i < C; ++i)
-        if (c * C + i > 0) dst[o0 + i * P] = (T)v[i];
+    for (int i = 0; i < C; ++i) {
+        const int j = c * C + i - 1;
+        if (SRC == YSRC_BOTH ? j >= out0 && j < out1 : j >= 0) dst[o0 + i * P] = (T)v[i];
+    }
 }
 
-template <class T, int C, int TX, int LPM, int E, bool SYNTH>
+template <class T, int C, int TX, int LPM, int E, int SRC>
 cudaError_t launch_ys(const Geom& g, T* data, SlabMap map, int nslabs, const SpecParams& sp, T* out,
-                      const BtSynth& bs, cudaStream_t st) {
-    const size_t smem = SYNTH ? (size_t)g.nx * sizeof(double) : 0;
+                      const YSource& ys, cudaStream_t st) {
+    const size_t smem = SRC == YSRC_EDGES || SRC == YSRC_UNIT ? (size_t)g.nx * sizeof(double) : 0;
     const int threads = (TX * (g.ny / C > LPM ? g.ny / C : LPM) + 31) & ~31;
-    return launch_k(y_solve_kernel<T, C, TX, LPM, E, SYNTH>, dim3((g.n1 + TX - 1) / TX, nslabs), dim3(threads), smem,
-                    st, data, map, g, sp, out, bs);
+    return launch_k(y_solve_kernel<T, C, TX, LPM, E, SRC>, dim3((g.n1 + TX - 1) / TX, nslabs), dim3(threads), smem,
+                    st, data, map, g, sp, out, ys);
 }
 
 // Rows per thread and lanes per mode by ny (a multiple of 8 from 32 to 2048).
@@ -294,24 +360,24 @@ cudaError_t launch_ys(const Geom& g, T* data, SlabMap map, int nslabs, const Spe
 // take 156 µs for the six solves of a 1024² x 5-level step against 167.
 // TX = 8 modes (64-byte rows in FP64): 4 modes are 1-2% slower at 512² and
 // 1024², the loads being half as wide.
-template <class T, bool SYNTH>
+template <class T, int SRC>
 cudaError_t launch_ys_t(const Geom& g, T* data, SlabMap map, int nslabs, const SpecParams& sp, T* out,
-                        const BtSynth& bs, cudaStream_t st) {
+                        const YSource& ys, cudaStream_t st) {
     constexpr int TX = 8;
     const int ny = g.ny;
     if (ny % 8 || ny < 32 || ny > 2048 || (ny > 512 && ny % 64)) return cudaErrorInvalidValue;
-    if (ny <= 64) return launch_ys<T, 8, TX, 8, 1, SYNTH>(g, data, map, nslabs, sp, out, bs, st);
-    if (ny <= 128) return launch_ys<T, 8, TX, 16, 1, SYNTH>(g, data, map, nslabs, sp, out, bs, st);
-    if (ny <= 256) return launch_ys<T, 8, TX, 32, 1, SYNTH>(g, data, map, nslabs, sp, out, bs, st);
+    if (ny <= 64) return launch_ys<T, 8, TX, 8, 1, SRC>(g, data, map, nslabs, sp, out, ys, st);
+    if (ny <= 128) return launch_ys<T, 8, TX, 16, 1, SRC>(g, data, map, nslabs, sp, out, ys, st);
+    if (ny <= 256) return launch_ys<T, 8, TX, 32, 1, SRC>(g, data, map, nslabs, sp, out, ys, st);
     if (ny <= 512) {
         if (ny % 16) return cudaErrorInvalidValue;       // two chunks per scan lane
-        return launch_ys<T, 8, TX, 32, 2, SYNTH>(g, data, map, nslabs, sp, out, bs, st);
+        return launch_ys<T, 8, TX, 32, 2, SRC>(g, data, map, nslabs, sp, out, ys, st);
     }
     if (ny <= 1024) {
         if (ny % 32) return cudaErrorInvalidValue;
-        return launch_ys<T, 16, TX, 32, 2, SYNTH>(g, data, map, nslabs, sp, out, bs, st);
+        return launch_ys<T, 16, TX, 32, 2, SRC>(g, data, map, nslabs, sp, out, ys, st);
     }
-    return launch_ys<T, 16, TX, 32, 4, SYNTH>(g, data, map, nslabs, sp, out, bs, st);
+    return launch_ys<T, 16, TX, 32, 4, SRC>(g, data, map, nslabs, sp, out, ys, st);
 }
 
 }  // namespace
@@ -319,15 +385,27 @@ cudaError_t launch_ys_t(const Geom& g, T* data, SlabMap map, int nslabs, const S
 cudaError_t launch_y_solve(const Geom& g, void* data, SlabMap map, int nslabs, const SpecParams& sp, cudaStream_t st) {
     if (nslabs <= 0) return cudaSuccess;
     if (sp.f32)
-        return launch_ys_t<float, false>(g, static_cast<float*>(data), map, nslabs, sp, nullptr, BtSynth{}, st);
-    return launch_ys_t<double, false>(g, static_cast<double*>(data), map, nslabs, sp, nullptr, BtSynth{}, st);
+        return launch_ys_t<float, YSRC_DATA>(g, static_cast<float*>(data), map, nslabs, sp, nullptr, YSource{}, st);
+    return launch_ys_t<double, YSRC_DATA>(g, static_cast<double*>(data), map, nslabs, sp, nullptr, YSource{}, st);
 }
 
 cudaError_t launch_y_solve_edges(const Geom& g, void* out, SlabMap map, int nslabs, const SpecParams& sp,
                                  const BtSynth& bs, cudaStream_t st) {
     if (nslabs <= 0) return cudaSuccess;
-    if (sp.f32) return launch_ys_t<float, true>(g, nullptr, map, nslabs, sp, static_cast<float*>(out), bs, st);
-    return launch_ys_t<double, true>(g, nullptr, map, nslabs, sp, static_cast<double*>(out), bs, st);
+    YSource ys;
+    ys.edges = bs;
+    if (sp.f32) return launch_ys_t<float, YSRC_EDGES>(g, nullptr, map, nslabs, sp, static_cast<float*>(out), ys, st);
+    return launch_ys_t<double, YSRC_EDGES>(g, nullptr, map, nslabs, sp, static_cast<double*>(out), ys, st);
+}
+
+cudaError_t launch_y_solve_both(const Geom& g, double* data, SlabMap map, int nslabs, const SpecParams& sp,
+                                const YSource& ys, cudaStream_t st) {
+    return launch_ys_t<double, YSRC_BOTH>(g, data, map, nslabs, sp, nullptr, ys, st);
+}
+
+cudaError_t launch_y_solve_unit(const Geom& g, double* data, SlabMap map, int nslabs, const SpecParams& sp,
+                                const YSource& ys, cudaStream_t st) {
+    return launch_ys_t<double, YSRC_UNIT>(g, data, map, nslabs, sp, nullptr, ys, st);
 }
 
 }  // namespace ibpm
