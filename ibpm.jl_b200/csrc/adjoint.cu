@@ -290,65 +290,72 @@ cudaError_t launch_adj_xb(const Geom& g, const BodyDev& b, const AdjXbArgs& a, c
 }
 
 // y = Aᵀ x, A row-major n×n (the transpose of F̃b = B⁻¹ F): 32 columns per
-// block, the rows split over 8 warps, partial sums added in a fixed order.
-__global__ void gemv_t_kernel(const double* __restrict__ A, const double* __restrict__ x, double* y, int n) {
+// block, the rows split over 32 warps (few blocks at these sizes: with 8 warps a
+// thread walked n/8 rows, 16 µs at n = 402 against 7.5), partial sums added in a
+// fixed order.
+__global__ void __launch_bounds__(1024) gemv_t_kernel(const double* __restrict__ A, const double* __restrict__ x,
+                                                      double* y, int n) {
     pdl_wait();
     pdl_trigger();
-    __shared__ double part[8][32];
-    const int c = blockIdx.x * 32 + (threadIdx.x & 31);
+    __shared__ double part[32][33];
+    const int lane = threadIdx.x & 31, c = blockIdx.x * 32 + lane;
     const int w = threadIdx.x >> 5;
     double acc = 0.0;
-    if (c < n)
-        for (int r = w; r < n; r += 8) acc += A[(long long)r * n + c] * x[r];
-    part[w][threadIdx.x & 31] = acc;
-    __syncthreads();
-    if (w == 0 && c < n) {
-        double s = 0.0;
-        for (int u = 0; u < 8; ++u) s += part[u][threadIdx.x];
-        y[c] = s;
+    if (c < n) {
+#pragma unroll 8
+        for (int r = w; r < n; r += 32) acc += A[(long long)r * n + c] * x[r];
     }
+    part[w][lane] = acc;
+    __syncthreads();
+    // warp w adds the 32 partial sums of column w of the block
+    const double s = warp_sum_d(part[lane][w]);
+    const int col = blockIdx.x * 32 + w;
+    if (lane == 0 && col < n) y[col] = s;
 }
 
 cudaError_t launch_gemv_t(const double* A, const double* x, double* y, int n, cudaStream_t st) {
-    return launch_k(gemv_t_kernel, dim3((n + 31) / 32), dim3(256), 0, st, A, x, y, n);
+    return launch_k(gemv_t_kernel, dim3((n + 31) / 32), dim3(1024), 0, st, A, x, y, n);
 }
 
 // q̄s = E' F̄ on the touched level-1 flux points (reg!, interface-coupling.jl:
-// 99-119, contributors in ascending component order), and the sums of q̄s over
-// the x and y fluxes (the adjoint of the uniform base flux of E(qs + q0)),
-// accumulated into acc[0..1].  One block.
-__global__ void adj_Et_kernel(BodyDev b, Geom g, const double* __restrict__ Fbar, double* qsb, double* acc) {
+// 99-119, contributors in ascending component order), one thread per point, and
+// the sums of q̄s over the x and y fluxes (the adjoint of the uniform base flux
+// of E(qs + q0)), added to the block's own slot of acc (fixed order over steps).
+// The lists are constants: their bounds are read before the dependency wait.  As
+// one block of 1024 threads it took 56 µs of an adjoint step at 256² with 201
+// points (6 500 rows), in blocks over all rows 12.
+constexpr int kEtThreads = 128;
+
+__global__ void __launch_bounds__(kEtThreads) adj_Et_kernel(BodyDev b, Geom g, const double* __restrict__ Fbar,
+                                                            double* qsb, double* acc) {
+    __shared__ double red[2][kEtThreads / 32];
+    const int r = blockIdx.x * kEtThreads + threadIdx.x;
+    const bool on = r < b.n_et_rows;
+    const int e0 = on ? b.et_ptr[r] : 0, e1 = on ? b.et_ptr[r + 1] : 0, f = on ? b.et_flux[r] : 0;
     pdl_wait();
     pdl_trigger();
-    __shared__ double red[2][1024];
-    double sx = 0.0, sy = 0.0;
-    for (int r = threadIdx.x; r < b.n_et_rows; r += blockDim.x) {
-        double v = 0.0;
-        for (int e = b.et_ptr[r]; e < b.et_ptr[r + 1]; ++e) v += b.w[b.et_w[e]] * Fbar[b.et_k[e]];
-        const int f = b.et_flux[r];
-        qsb[f] = v;
-        if (f < g.nu) sx += v;
-        else sy += v;
+    double v = 0.0;
+#pragma unroll 8
+    for (int e = e0; e < e1; ++e) v += b.w[b.et_w[e]] * Fbar[b.et_k[e]];
+    if (on) qsb[f] = v;
+    const double sx = warp_sum_d(on && f < g.nu ? v : 0.0), sy = warp_sum_d(on && f >= g.nu ? v : 0.0);
+    if ((threadIdx.x & 31) == 0) {
+        red[0][threadIdx.x >> 5] = sx;
+        red[1][threadIdx.x >> 5] = sy;
     }
-    red[0][threadIdx.x] = sx;
-    red[1][threadIdx.x] = sy;
     __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) {
-            red[0][threadIdx.x] += red[0][threadIdx.x + s];
-            red[1][threadIdx.x] += red[1][threadIdx.x + s];
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        acc[0] += red[0][0];
-        acc[1] += red[1][0];
+    if (threadIdx.x < 2) {
+        double s = 0.0;
+        for (int u = 0; u < kEtThreads / 32; ++u) s += red[threadIdx.x][u];
+        acc[2 * blockIdx.x + threadIdx.x] += s;
     }
 }
 
+int adj_Et_blocks(const BodyDev& b) { return (b.n_et_rows + kEtThreads - 1) / kEtThreads; }
+
 cudaError_t launch_adj_Et(const Geom& g, const BodyDev& b, const double* Fbar, double* qsb, double* acc,
                           cudaStream_t st) {
-    return launch_k(adj_Et_kernel, dim3(1), dim3(1024), 0, st, b, g, Fbar, qsb, acc);
+    return launch_k(adj_Et_kernel, dim3(adj_Et_blocks(b)), dim3(kEtThreads), 0, st, b, g, Fbar, qsb, acc);
 }
 
 // ---------------------------------------------------------------------------

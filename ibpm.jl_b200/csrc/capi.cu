@@ -119,7 +119,7 @@ struct ibpm_handle {
     double* qsb = nullptr;                 // q̄s (nq)
     double* Ft = nullptr; double* Fbar = nullptr;
     double* bcc = nullptr; double* bcv = nullptr;  // edge adjoints (mg·nbc each)
-    double* q0part = nullptr;              // [mg][blocks][2] + 2 (E' part)
+    double* q0part = nullptr;              // [mg][blocks][2], then [blocks][2] of the E' part
     double* stepw = nullptr;               // objective weight of each step
     int* adj_n = nullptr;
     double adj_wx = 0, adj_wy = 0;
@@ -1884,7 +1884,7 @@ static int adj_alloc(ibpm_handle* h, int k, int ncp, int nsteps) {
     for (double** b : bufs) if (*b) { cudaFree(*b); *b = nullptr; }
     if (h->adj_n) { cudaFree(h->adj_n); h->adj_n = nullptr; }
     int rc;
-    const long long nq0 = (long long)g.mg * adj_nlq_blocks(g) * 2 + 2;
+    const long long nq0 = 2ll * (g.mg * adj_nlq_blocks(g) + adj_Et_blocks(h->body));
     if ((rc = dalloc(h, &h->tapeG, (size_t)k * bs)) || (rc = dalloc(h, &h->tapeq, (size_t)k * qs)) ||
         (rc = dalloc(h, &h->ck, (size_t)(ncp + 1) * ckd)) || (rc = dalloc(h, &h->Gb, bs)) ||
         (rc = dalloc(h, &h->qb, qs)) || (rc = dalloc(h, &h->Nb[0], bs)) || (rc = dalloc(h, &h->Nb[1], bs)) ||
@@ -1990,7 +1990,7 @@ extern "C" int ibpm_adjoint_run(ibpm_handle* h, int32_t nsteps, int32_t k_checkp
     // ---- reverse sweep: recompute each segment into the tape, then adjoint steps
     for (double* p : {h->Gb, h->Nb[0], h->Nb[1]}) CK(cudaMemsetAsync(p, 0, sizeof(double) * bs, h->st));
     CK(cudaMemsetAsync(h->qb, 0, sizeof(double) * qs, h->st));
-    const long long nq0 = (long long)mg * adj_nlq_blocks(g) * 2 + 2;
+    const long long nq0 = 2ll * (mg * adj_nlq_blocks(g) + adj_Et_blocks(h->body));
     CK(cudaMemsetAsync(h->q0part, 0, sizeof(double) * nq0, h->st));
     if (h->adj_xb) CK(cudaMemsetAsync(h->gxb, 0, sizeof(double) * h->nf, h->st));
     const int last = nsteps - 1;
@@ -2048,7 +2048,8 @@ extern "C" int ibpm_adjoint_run(ibpm_handle* h, int32_t nsteps, int32_t k_checkp
         for (int l = 0; l < mg; ++l) {
             double sx = 0.0, sy = 0.0;
             for (int b = 0; b < nb; ++b) { sx += part[2 * ((size_t)l * nb + b)]; sy += part[2 * ((size_t)l * nb + b) + 1]; }
-            if (l == 0) { sx += part[nq0 - 2]; sy += part[nq0 - 1]; }
+            if (l == 0)
+                for (size_t b = 2 * (size_t)mg * nb; b < part.size(); b += 2) { sx += part[b]; sy += part[b + 1]; }
             const double hc = h->h * std::ldexp(1.0, l), a = h->incl;
             d += sx * (-h->Ux * std::sin(a) - h->Uy * std::cos(a)) * hc;
             d += sy * (h->Ux * std::cos(a) - h->Uy * std::sin(a)) * hc;

@@ -520,6 +520,7 @@ cudaError_t launch_zero_centre(const Geom& g, double* G, cudaStream_t st);
 cudaError_t launch_adj_E_rotT(const Geom& g, const BodyDev& b, const double* W, double wx, double wy,
                               const double* stepw, const int* adj_n, double* Ft, cudaStream_t st);
 cudaError_t launch_gemv_t(const double* A, const double* x, double* y, int n, cudaStream_t st);
+int adj_Et_blocks(const BodyDev& b);   // acc holds two sums per block
 cudaError_t launch_adj_Et(const Geom& g, const BodyDev& b, const double* Fbar, double* qsb, double* acc,
                           cudaStream_t st);
 // Trial-step adjoint: see adjoint.cu.
