@@ -57,8 +57,7 @@ struct ibpm_handle {
     // body
     double* d_xb = nullptr; double* d_ds = nullptr; int* d_bidx = nullptr; double* d_w = nullptr;
     int* d_body_start = nullptr;
-    int* d_src_pts = nullptr; int* d_src_rows = nullptr; int* d_et_ptr = nullptr; int* d_et_k = nullptr;
-    int* d_et_w = nullptr; int* d_et_flux = nullptr;
+    int* d_lists = nullptr;                      // the lists of E' and C'E', one allocation
     BodyDev body{};
     int win_y0 = 0, win_y1 = 0;            // slab rows of ψ that E reads (fixed bodies), [y0, y1)
     bool win_inside = false;               // … none of them through the level's edge values
@@ -884,52 +883,9 @@ static int build_coupling(ibpm_handle* h, const ibpm_problem_desc* d) {
         h->win_y1 = std::min(g.n2, *my.second + 6);
         h->win_inside = *mx.first - 6 >= 2 && *mx.second + 6 <= g.nx - 1 && *my.first - 6 >= 2 && *my.second + 6 <= g.ny - 1;
     }
-    // E' as CSR over touched flux points, contributors in ascending component order.
-    std::map<int, std::vector<std::pair<int, int>>> rows;  // flux index -> (kk, widx)
-    for (int kk = 0; kk < h->nf; ++kk) {
-        const int comp = kk / nb, k = kk % nb;
-        const int bx = bidx[k], by = bidx[nb + k];
-        for (int l = 0; l < 13; ++l)
-            for (int m = 0; m < 13; ++m) {
-                const int I = bx + l - 6, J = by + m - 6;
-                const int f = comp == 0 ? (I - 1) + (J - 1) * (g.nx + 1) : g.nu + (I - 1) + (J - 1) * g.nx;
-                rows[f].push_back({kk, (kk * 13 + l) * 13 + m});
-            }
-    }
-    std::vector<int> et_ptr, et_k, et_w, et_flux;
-    std::map<int, int> row_of;
-    et_ptr.push_back(0);
-    for (auto& kv : rows) {
-        row_of[kv.first] = (int)et_ptr.size() - 1;
-        et_flux.push_back(kv.first);
-        for (auto& e : kv.second) { et_k.push_back(e.first); et_w.push_back(e.second); }
-        et_ptr.push_back((int)et_k.size());
-    }
-    // Γ points whose rot! stencil touches a regularised flux: Γ(i0, j0) uses
-    // qx[i0+2, j0+1], qx[i0+2, j0+2], qy[i0+2, j0+2], qy[i0+1, j0+2] (1-based).
-    auto fx = [&](int I, int J) { return (I - 1) + (J - 1) * (g.nx + 1); };
-    auto fy = [&](int I, int J) { return g.nu + (I - 1) + (J - 1) * g.nx; };
-    std::vector<int> src_pts, src_rows;
-    for (int j0 = 0; j0 < g.n2; ++j0)
-        for (int i0 = 0; i0 < g.n1; ++i0) {
-            const int f4[4] = {fx(i0 + 2, j0 + 1), fx(i0 + 2, j0 + 2), fy(i0 + 2, j0 + 2), fy(i0 + 1, j0 + 2)};
-            int r4[4];
-            bool any = false;
-            for (int r = 0; r < 4; ++r) {
-                auto it = row_of.find(f4[r]);
-                r4[r] = it == row_of.end() ? -1 : it->second;
-                any |= r4[r] >= 0;
-            }
-            if (!any) continue;
-            src_pts.push_back(j0 * g.P + i0);
-            for (int r = 0; r < 4; ++r) src_rows.push_back(r4[r]);
-        }
     int rc;
     if ((rc = dalloc(h, &h->d_xb, 2 * nb)) || (rc = dalloc(h, &h->d_ds, nb)) || (rc = dalloc(h, &h->d_bidx, 2 * nb)) ||
-        (rc = dalloc(h, &h->d_w, (size_t)h->nf * 169)) || (rc = dalloc(h, &h->d_body_start, h->nbodies + 1)) ||
-        (rc = dalloc(h, &h->d_src_pts, src_pts.size())) || (rc = dalloc(h, &h->d_src_rows, src_rows.size())) ||
-        (rc = dalloc(h, &h->d_et_ptr, et_ptr.size())) || (rc = dalloc(h, &h->d_et_k, et_k.size())) ||
-        (rc = dalloc(h, &h->d_et_w, et_w.size())) || (rc = dalloc(h, &h->d_et_flux, et_flux.size())))
+        (rc = dalloc(h, &h->d_w, (size_t)h->nf * 169)) || (rc = dalloc(h, &h->d_body_start, h->nbodies + 1)))
         return rc;
     auto up = [&](void* dst, const void* src, size_t bytes) {
         return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, h->st);
@@ -938,21 +894,40 @@ static int build_coupling(ibpm_handle* h, const ibpm_problem_desc* d) {
     CK(up(h->d_ds, d->ds, sizeof(double) * nb));
     CK(up(h->d_bidx, bidx.data(), sizeof(int) * 2 * nb));
     CK(up(h->d_body_start, h->body_start.data(), sizeof(int) * (h->nbodies + 1)));
-    if (!src_pts.empty()) {
-        CK(up(h->d_src_pts, src_pts.data(), sizeof(int) * src_pts.size()));
-        CK(up(h->d_src_rows, src_rows.data(), sizeof(int) * src_rows.size()));
-    }
-    CK(up(h->d_et_ptr, et_ptr.data(), sizeof(int) * et_ptr.size()));
-    CK(up(h->d_et_k, et_k.data(), sizeof(int) * et_k.size()));
-    CK(up(h->d_et_w, et_w.data(), sizeof(int) * et_w.size()));
-    CK(up(h->d_et_flux, et_flux.data(), sizeof(int) * et_flux.size()));
-    CK(cudaStreamSynchronize(h->st));  // host vectors go out of scope
+    // the lists of E' and C'E': counted, then written to one allocation of their size
+    char* scratch = nullptr;
+    if ((rc = dalloc(h, &scratch, coupling_scratch_bytes(g, nb)))) return rc;
+    CouplingLists c{};
+    int n_src = 0;
+    auto lists = [&]() -> int {
+        unsigned long long tot[2];
+        CK(launch_coupling_count(g, h->d_bidx, nb, scratch, h->st));
+        CK(cudaMemcpyAsync(tot, scratch, sizeof(tot), cudaMemcpyDeviceToHost, h->st));
+        CK(cudaStreamSynchronize(h->st));
+        const size_t n_et = (size_t)h->nf * 169;
+        c.n_rows = (int)(tot[0] >> 32);
+        n_src = (int)tot[1];
+        int rc = dalloc(h, &h->d_lists, 2 * n_et + 2 * (size_t)c.n_rows + 1 + 5 * (size_t)n_src);
+        if (rc) return rc;
+        c.et_k = h->d_lists;
+        c.et_w = c.et_k + n_et;
+        c.et_flux = c.et_w + n_et;
+        c.et_ptr = c.et_flux + c.n_rows;
+        c.src_pts = c.et_ptr + c.n_rows + 1;
+        c.src_rows = c.src_pts + n_src;
+        CK(launch_coupling_lists(g, h->d_bidx, nb, scratch, c, h->st));
+        CK(cudaStreamSynchronize(h->st));
+        return IBPM_OK;
+    };
+    rc = lists();
+    cudaFree(scratch);
+    if (rc) return rc;
     BodyDev& b = h->body;
     b.nb = nb; b.nf = h->nf; b.nbodies = h->nbodies;
     b.xb = h->d_xb; b.ds = h->d_ds; b.bidx = h->d_bidx; b.w = h->d_w; b.body_start = h->d_body_start;
-    b.n_src = (int)src_pts.size(); b.src_pts = h->d_src_pts; b.src_rows = h->d_src_rows;
-    b.et_ptr = h->d_et_ptr; b.et_k = h->d_et_k; b.et_w = h->d_et_w;
-    b.n_et_rows = (int)et_flux.size(); b.et_flux = h->d_et_flux;
+    b.n_src = n_src; b.src_pts = c.src_pts; b.src_rows = c.src_rows;
+    b.et_ptr = c.et_ptr; b.et_k = c.et_k; b.et_w = c.et_w;
+    b.n_et_rows = c.n_rows; b.et_flux = c.et_flux;
     CK(launch_weights(g, d->h, d->offx, d->offy, b, h->st));
     return IBPM_OK;
 }
@@ -1024,7 +999,7 @@ static void free_handle(ibpm_handle* h) {
     for (void* p : adj) if (p) cudaFree(p);
     void* ptrs[] = {h->G[0], h->G[1], h->Nl[0], h->Nl[1], h->psi, h->q, h->rhs, h->Gsrc, h->F, h->Fb,
                     h->Binv, h->nonlin1_shadow, h->d_xb, h->d_ds, h->d_bidx, h->d_w, h->d_body_start,
-                    h->d_src_pts, h->d_src_rows, h->d_et_ptr, h->d_et_k, h->d_et_w, h->d_et_flux, h->hist,
+                    h->d_lists, h->hist,
                     h->counter};
     for (void* p : ptrs) if (p) cudaFree(p);
     if (h->flush_buf) cudaFree(h->flush_buf);

@@ -464,6 +464,16 @@ struct BodyDev {
     int n_et_rows;          // touched flux points
     const int* et_flux;     // [n_et_rows] level-1 flux index of each CSR row
 };
+// Building the lists (coupling.cu): a count, whose totals (rows << 32 | contributors,
+// and source points) are the first two words of the scratch, then the lists.
+struct CouplingLists {
+    int *et_ptr, *et_k, *et_w, *et_flux, *src_pts, *src_rows;
+    int n_rows;
+};
+size_t coupling_scratch_bytes(const Geom& g, int nb);
+cudaError_t launch_coupling_count(const Geom& g, const int* bidx, int nb, void* scratch, cudaStream_t st);
+cudaError_t launch_coupling_lists(const Geom& g, const int* bidx, int nb, void* scratch, const CouplingLists& c,
+                                  cudaStream_t st);
 cudaError_t launch_weights(const Geom& g, double h, double offx, double offy,
                            const BodyDev& b, cudaStream_t st);
 // E (C ψ + q0) of level 1 from ψ (its slab, the next level's behind it); fixed:
