@@ -33,17 +33,9 @@ namespace ibpm {
 // MOV: a moving grid's per-face base flux (MovingFlux) instead of q0x, q0y.
 // GRP: the simulations of a batch group, blockIdx.z = simulation · mg + level,
 // each with its own arguments in ga[simulation] (its fields, coefficients).
-template <bool LIN, bool MOV, bool GRP = false>
-__global__ void __launch_bounds__(256) trial_rhs_kernel(const __grid_constant__ RhsArgs a0,
-                                                        const RhsArgs* __restrict__ ga, Geom g) {
-    pdl_wait();
-    pdl_trigger();
-    const RhsArgs& a = GRP ? ga[blockIdx.z / g.mg] : a0;
-    const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j0 = blockIdx.y * blockDim.y + threadIdx.y;
-    const int lev = GRP ? (int)(blockIdx.z % g.mg) : (int)blockIdx.z;
+template <bool LIN, bool MOV>
+__device__ __forceinline__ void trial_point(const RhsArgs& a, const Geom& g, int lev, int i0, int j0) {
     const int nx = g.nx, ny = g.ny, n1 = g.n1, n2 = g.n2, P = g.P;
-    if (i0 >= n1 || j0 >= n2) return;
     const double* G = a.G + a.Gmap.off(lev);
     const double* q = a.q + (long long)lev * g.nq;
     const int o = j0 * P + i0;                           // a level is below 2^31 values
@@ -117,17 +109,117 @@ __global__ void __launch_bounds__(256) trial_rhs_kernel(const __grid_constant__ 
     a.rhs[oo] = ((AG + a.b1dt * N) + a.b2dt * Np) + rbc;
 }
 
+template <bool LIN, bool MOV, bool GRP = false>
+__global__ void __launch_bounds__(256) trial_rhs_kernel(const __grid_constant__ RhsArgs a0,
+                                                        const RhsArgs* __restrict__ ga, Geom g) {
+    pdl_wait();
+    pdl_trigger();
+    const RhsArgs& a = GRP ? ga[blockIdx.z / g.mg] : a0;
+    const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j0 = blockIdx.y * blockDim.y + threadIdx.y;
+    const int lev = GRP ? (int)(blockIdx.z % g.mg) : (int)blockIdx.z;
+    if (i0 >= g.n1 || j0 >= g.n2) return;
+    trial_point<LIN, MOV>(a, g, lev, i0, j0);
+}
+
+// The same for 2 × 2 points per thread (fixed grid, not linearised): 40 values read
+// for 4 points instead of 56, most in aligned pairs, so 30 load instructions instead
+// of 56.  Points on the rim, the columns 0, 1, n1 − 1 and the rows 0, 1, n2 − 1, are
+// the business of extra blocks, one point per thread, so that no warp takes both
+// paths (inside the tiles' blocks they cost 4 µs of a step at any size).  1023² x 5
+// levels: 65 -> 43 µs, of which the bytes take 39; 511² x 5 22 -> 14.
+template <bool GRP>
+__global__ void __launch_bounds__(256) trial_rhs_tile_kernel(const __grid_constant__ RhsArgs a0,
+                                                             const RhsArgs* __restrict__ ga, Geom g) {
+    pdl_wait();
+    pdl_trigger();
+    const RhsArgs& a = GRP ? ga[blockIdx.z / g.mg] : a0;
+    const int lev = GRP ? (int)(blockIdx.z % g.mg) : (int)blockIdx.z;
+    const int nx = g.nx, n1 = g.n1, n2 = g.n2, P = g.P;
+    const int rim0 = (n2 + 15) / 16;                     // the blocks of tiles are rows 0 … rim0 − 1
+    if ((int)blockIdx.y >= rim0) {
+        // the columns 0, 1, n1 − 1, then what is left of the rows 0, 1, n2 − 1
+        const int t = ((blockIdx.y - rim0) * gridDim.x + blockIdx.x) * 256 + threadIdx.y * 32 + threadIdx.x;
+        const int u = t - 3 * n2;
+        if (u >= 3 * (n1 - 3)) return;
+        const int s = t < 3 * n2 ? t / n2 : u / (n1 - 3);
+        const int i = t < 3 * n2 ? (s < 2 ? s : n1 - 1) : 2 + u - s * (n1 - 3);
+        const int j = t < 3 * n2 ? t - s * n2 : (s < 2 ? s : n2 - 1);
+        trial_point<false, false>(a, g, lev, i, j);
+        return;
+    }
+    const int i0 = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
+    const int j0 = 2 * (blockIdx.y * blockDim.y + threadIdx.y);
+    if (i0 == 0 || i0 >= n1 - 1 || j0 == 0 || j0 >= n2 - 1) return;
+    // i0, P, nx, the level's and the y-faces' offsets are even: pairs are aligned
+    auto two = [](const double* p) { return *reinterpret_cast<const double2*>(p); };
+    const long long oo = a.Gmap.off(lev) + j0 * P + i0;
+    const double* G = a.G + oo;
+    const double* fx = a.q + (long long)lev * g.nq + j0 * (nx + 1) + i0;
+    const double* fy = a.q + (long long)lev * g.nq + g.nu + j0 * nx + i0;
+    double2 c[4], y2[4], Np[2];
+    double w[2], e[2], x[3][4], y1[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        c[r] = two(G + (r - 1) * P);
+        y2[r] = two(fy + r * nx);
+        y1[r] = fy[r * nx + 2];
+    }
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) x[r][k] = fx[r * (nx + 1) + k];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        w[r] = G[r * P - 1];
+        e[r] = G[r * P + 2];
+        Np[r] = two(a.Nprev + oo + r * P);
+    }
+    const double bx = 2.0 * a.q0x[lev], by = 2.0 * a.q0y[lev], sc = a.nl_scale[lev], cl = a.c_lap[lev];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        double N[2], R[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const double gc = k ? c[r + 1].y : c[r + 1].x, gs = k ? c[r].y : c[r].x, gn = k ? c[r + 2].y : c[r + 2].x;
+            const double gw = k ? c[r + 1].x : w[r], ge = k ? e[r] : c[r + 1].y;
+            const double Qw = (x[r + 1][k] + x[r][k]) + bx, Qe = (x[r + 1][k + 2] + x[r][k + 2]) + bx;
+            const double Qs = (k ? y1[r] + y2[r].y : y2[r].y + y2[r].x) + by;
+            const double Qn = (k ? y1[r + 2] + y2[r + 2].y : y2[r + 2].y + y2[r + 2].x) + by;
+            N[k] = ((Qs * gs - Qn * gn) + (Qw * gw - Qe * ge)) * sc;
+            const double AG = gc + cl * ((((ge + gw) + gn) + gs) - 4.0 * gc);
+            R[k] = (AG + a.b1dt * N[k]) + a.b2dt * (k ? Np[r].y : Np[r].x);
+        }
+        *reinterpret_cast<double2*>(a.Nnew + oo + r * P) = make_double2(N[0], N[1]);
+        *reinterpret_cast<double2*>(a.rhs + oo + r * P) = make_double2(R[0], R[1]);
+    }
+}
+
+// From 2^19 points of a simulation on, the tiles are the faster (512² x 3 levels
+// 137.5 -> 136.6 µs per step, x 5 177.2 -> 174.0, 1024² x 3 326 -> 313, x 5 491 ->
+// 471); below, the step loses up to 1 µs to them (64² x 3 60.5 -> 61.5, 256² x 4
+// 100.3 -> 101.2, 400x200 x 5 even): too few threads, each with a longer chain.
+// The size of one simulation decides, also in a group: a member's results do not
+// depend on its group.
+static bool trial_tiled(const Geom& g) { return (long long)g.n1 * g.n2 * g.mg >= 1 << 19; }
+static dim3 trial_tiles(const Geom& g, int nsim) {
+    const int bx = (g.n1 + 63) / 64, rim = (3 * g.n2 + 3 * (g.n1 - 3) + 255) / 256;
+    return dim3(bx, (g.n2 + 15) / 16 + (rim + bx - 1) / bx, nsim * g.mg);
+}
+
 cudaError_t launch_trial_rhs(const Geom& g, const RhsArgs& a, cudaStream_t st) {
     dim3 blk(32, 8);
     dim3 grid((g.n1 + 31) / 32, (g.n2 + 7) / 8, a.mg);
     const RhsArgs* none = nullptr;
     if (a.GB) return launch_k(trial_rhs_kernel<true, false>, grid, blk, 0, st, a, none, g);
     if (a.mv.tab) return launch_k(trial_rhs_kernel<false, true>, grid, blk, 0, st, a, none, g);
+    if (trial_tiled(g)) return launch_k(trial_rhs_tile_kernel<false>, trial_tiles(g, 1), blk, 0, st, a, none, g);
     return launch_k(trial_rhs_kernel<false, false>, grid, blk, 0, st, a, none, g);
 }
 
 cudaError_t launch_trial_rhs_group(const Geom& g, const RhsArgs& a0, const RhsArgs* ga, int nsim, cudaStream_t st) {
     dim3 blk(32, 8);
+    if (trial_tiled(g)) return launch_k(trial_rhs_tile_kernel<true>, trial_tiles(g, nsim), blk, 0, st, a0, ga, g);
     dim3 grid((g.n1 + 31) / 32, (g.n2 + 7) / 8, nsim * g.mg);
     return launch_k(trial_rhs_kernel<false, false, true>, grid, blk, 0, st, a0, ga, g);
 }
