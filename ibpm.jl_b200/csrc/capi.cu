@@ -870,7 +870,8 @@ static int build_coupling(ibpm_handle* h, const ibpm_problem_desc* d) {
         bidx[k] = (int)std::floor((d->xb[k] + d->offx) / d->h);
         bidx[nb + k] = (int)std::floor((d->xb[nb + k] + d->offy) / d->h);
         const int bx = bidx[k], by = bidx[nb + k];
-        if (bx - 6 < 1 || bx + 6 > g.nx || by - 6 < 1 || by + 6 > g.ny)
+        // written so that a point that is no number (INT_MIN) is refused too
+        if (bx < 7 || bx > g.nx - 6 || by < 7 || by > g.ny - 6)
             return fail(h, IBPM_ERR_INVALID, "body point " + std::to_string(k) +
                                                  ": the 13x13 regularisation stencil leaves the finest grid");
     }
