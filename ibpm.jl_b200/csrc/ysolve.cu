@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(TX * LPM * E, ys_min_blocks<C, TX * LPM * E>()
     __shared__ double sV[TX * LC], sW[TX * LC];
     __shared__ double sC[4 * TX];                        // r, κ·scale, 1/(1−r^{2ny}), 1−r² of each mode
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    double* sn = reinterpret_cast<double*>(smem_raw);    // edges, unit: sin(π t/nx), t < nx; edges: 4 folded rows
+    double* sn = reinterpret_cast<double*>(smem_raw);    // edges, unit: sin(π t/nx), t < nx
     const int P = g.P, n1 = g.n1, nx = g.nx, nc = g.ny / C;
     const int tid = threadIdx.x, x = tid % TX, c = tid / TX;
     const bool own = c < nc;                             // the block is padded to whole warps
@@ -144,41 +144,24 @@ __global__ void __launch_bounds__(TX * LPM * E, ys_min_blocks<C, TX * LPM * E>()
     if constexpr (SRC == YSRC_EDGES) {
         const int ep = (2 * n1 + 2 * g.n2 + 3) & ~3;
         const double* e = ys.edges.e + ((long long)bt * g.mg + lev) * ep;
-        // The bottom and top rows folded about the middle, S(nx − i, k) =
-        // (−1)^{k+1} S(i, k): the sums for odd k, then the differences.  Read once by
-        // the block, beside the loads of the side columns, instead of by every
-        // thread for each of its terms, nx / nc rounds of two loads (two such
-        // launches per step: 64² x 3 levels 59.5 -> 57.5 µs, 200² x 3 82.0 -> 78.1,
-        // 400x200 x 5 114.8 -> 108.6, 512² x 5 173.9 -> 171.2, 1024² x 5 473 -> 458).
-        const int k = col + 1, nx2 = 2 * nx, H = nx / 2, HS = H + 4;
-        double* fold = sn + nx;
-        for (int i = tid; i < H; i += blockDim.x) {
-#pragma unroll
-            for (int row = 0; row < 2; ++row) {
-                const double p = __ldg(&e[row * n1 + i]), q = i < H - 1 ? __ldg(&e[row * n1 + n1 - 1 - i]) : 0.0;
-                fold[2 * row * HS + i] = p + q;
-                fold[(2 * row + 1) * HS + i] = p - q;
-            }
-        }
-        side(e + 2 * n1, e + 2 * n1 + g.n2, 2.0 * sinpix(k % nx2));
-        __syncthreads();
-        // this thread's share of the sine sums
+        const int k = col + 1, nx2 = 2 * nx;
+        // this thread's share of the sine sums of the bottom and top rows
         if (own) {
-            const double* fb = fold + (k & 1 ? 0 : HS);
             double pb = 0.0, pt = 0.0;
             int t = ((c + 1) * k) % nx2;
             const int dt = (nc * k) % nx2;
 #pragma unroll 4
-            for (int i = c; i < H; i += nc) {
+            for (int i = c; i < n1; i += nc) {
                 const double sv = sinpix(t);
-                pb = fma(sv, fb[i], pb);
-                pt = fma(sv, fb[2 * HS + i], pt);
+                pb = fma(sv, __ldg(&e[i]), pb);
+                pt = fma(sv, __ldg(&e[n1 + i]), pt);
                 t += dt;
                 if (t >= nx2) t -= nx2;
             }
             sV[x * LC + c] = pb;
             sW[x * LC + c] = pt;
         }
+        side(e + 2 * n1, e + 2 * n1 + g.n2, 2.0 * sinpix(k % nx2));
         __syncthreads();
         if (scans) {                                     // sums over the chunks
             double b = 0.0, tt = 0.0;
@@ -365,14 +348,7 @@ __global__ void __launch_bounds__(TX * LPM * E, ys_min_blocks<C, TX * LPM * E>()
 template <class T, int C, int TX, int LPM, int E, int SRC>
 cudaError_t launch_ys(const Geom& g, T* data, SlabMap map, int nslabs, const SpecParams& sp, T* out,
                       const YSource& ys, cudaStream_t st) {
-    // the sine table; for the edges also the folded bottom and top rows (16 kB more at
-    // nx = 1024; with the exchange arrays above 48 kB only at nx = 2048)
-    const size_t smem = sizeof(double) * (SRC == YSRC_EDGES ? 3 * g.nx + 16 : SRC == YSRC_UNIT ? g.nx : 0);
-    if (smem > 24 * 1024 + 128) {
-        cudaError_t e = cudaFuncSetAttribute(y_solve_kernel<T, C, TX, LPM, E, SRC>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    const size_t smem = SRC == YSRC_EDGES || SRC == YSRC_UNIT ? (size_t)g.nx * sizeof(double) : 0;
     const int threads = (TX * (g.ny / C > LPM ? g.ny / C : LPM) + 31) & ~31;
     return launch_k(y_solve_kernel<T, C, TX, LPM, E, SRC>, dim3((g.n1 + TX - 1) / TX, nslabs), dim3(threads), smem,
                     st, data, map, g, sp, out, ys);
