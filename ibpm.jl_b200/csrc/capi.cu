@@ -538,10 +538,11 @@ static int curl_levels(ibpm_handle* h, double* q, int qnlev) {
 
 // vort2flux! (FP64) of the handle's field G into h->psi (levels < nfull; the
 // coarser ones are left as they were) and q (levels < qnlev <= nfull; none
-// when only ψ is wanted); of a single level only its rows [y0, y1) where y1 > 0.
-// E of the trial vort2flux! reads ψ of level 1 around the bodies, and of level
-// 2 where a body's window meets the level's edge (trial_window); the final
-// vort2flux! recomputes every level.
+// when only ψ is wanted).  E of the trial vort2flux! reads ψ of level 1 around the
+// bodies, and of level 2 where a body's window meets the level's edge: then only
+// the rows [y0, y1) of the nfull levels, y1 > 0 (trial_window), by the plan of
+// single-slab launches, since a member of a group may need one level by itself
+// and two with the group.  The final vort2flux! recomputes every level.
 static int vort2flux_bt(ibpm_handle* h, double* G, double* q, int qnlev, int nfull, int y0 = 0, int y1 = 0) {
     const Geom& g = h->g;
     const int mg = g.mg, ns = h->gsim;
@@ -564,7 +565,9 @@ static int vort2flux_bt(ibpm_handle* h, double* G, double* q, int qnlev, int nfu
     c.in = h->rhs; c.in2 = h->btY; c.in_map = part; c.in2_map = part; c.out = h->psi; c.out_map = part;
     c.nslabs = nfull * ns; c.line0 = y1 > 0 ? y0 : 0; c.line1 = y1 > 0 ? y1 : g.n2;
     c.load = XLOAD_SUM; c.emit = XEMIT_STORE;
-    LAUNCH(K_DSTX, 24.0 * slab * nfull * ns * (c.line1 - c.line0) / g.n2, launch_dst_x(g, h->px, c, h->st));
+    DstPlan px = h->px;
+    if (y1 > 0) px.planN = px.plan1;
+    LAUNCH(K_DSTX, 24.0 * slab * nfull * ns * (c.line1 - c.line0) / g.n2, launch_dst_x(g, px, c, h->st));
     return qnlev > 0 ? curl_levels(h, q, qnlev) : IBPM_OK;
 }
 
@@ -621,9 +624,12 @@ static int trial_rhs(ibpm_handle* h, int p) {
 // member of the group being captured); else levels 1 and 2.  At 512² x 5 with a
 // unit cylinder this is 140 of 511 rows: the last x-pass takes 6 µs instead of
 // 10, the edge part's y-solve one level instead of two.
+// The x-pass transforms rows 2k and 2k + 1 as one complex line, so a row's last
+// bits depend on its partner: the window begins and ends on whole pairs, and a
+// member's rows have the same partners alone and in every group.
 struct TrialWindow { int nfull, y0, y1; };
 static TrialWindow trial_window(const ibpm_handle* h) {
-    TrialWindow w{std::min(2, h->g.mg), 0, 0};
+    const TrialWindow w{std::min(2, h->g.mg), 0, h->g.n2};
     if (h->bodies_moving) return w;
     int y0 = h->g.n2, y1 = 0;
     for (int i = 0; i < h->gsim; ++i) {
@@ -632,7 +638,7 @@ static TrialWindow trial_window(const ibpm_handle* h) {
         y0 = std::min(y0, m->win_y0);
         y1 = std::max(y1, m->win_y1);
     }
-    return TrialWindow{1, y0, y1};
+    return TrialWindow{1, y0 & ~1, std::min(h->g.n2, (y1 + 1) & ~1)};
 }
 
 // One step, reading the state from parity p and leaving it in parity p^1.
