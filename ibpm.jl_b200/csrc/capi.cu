@@ -1157,16 +1157,9 @@ static int state_transfer(ibpm_handle* h, const StatePiece* f, int nf, bool to_d
     for (int i = 0; i < nf && pack; ++i) {
         if (!f[i].host) continue;
         bytes += sizeof(double) * f[i].n;
-        // page-locked as a whole (first and last value), aligned
-        const double* last = f[i].host + (f[i].n - 1);
-        cudaPointerAttributes pa{}, pe{};
-        pack = bytes <= kPackBytes && reinterpret_cast<uintptr_t>(f[i].host) % sizeof(double) == 0 &&
-               cudaPointerGetAttributes(&pa, f[i].host) == cudaSuccess && pa.type == cudaMemoryTypeHost &&
-               cudaPointerGetAttributes(&pe, last) == cudaSuccess && pe.type == cudaMemoryTypeHost && pa.devicePointer &&
-               static_cast<double*>(pa.devicePointer) + (f[i].n - 1) == pe.devicePointer;
-        if (pack)
-            pk.piece[np++] = PackPiece{f[i].dev, static_cast<double*>(pa.devicePointer), f[i].n, f[i].slab ? g.n1 : 1,
-                                       f[i].slab ? g.P : 1};
+        double* mapped = bytes <= kPackBytes ? locked_host(f[i].host, f[i].n) : nullptr;
+        pack = mapped != nullptr;
+        if (pack) pk.piece[np++] = PackPiece{f[i].dev, mapped, f[i].n, f[i].slab ? g.n1 : 1, f[i].slab ? g.P : 1};
     }
     if (pack) {
         if (np) CK(launch_pack(pk, np, to_device, h->st));

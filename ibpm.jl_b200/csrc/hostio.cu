@@ -6,7 +6,10 @@
 // pieces: reading 64² x 3 levels (0.6 MB) 68 -> 29 µs, 200² x 3 (4 MB) 230 ->
 // 134 µs.  Above kPackBytes the copy engines are as fast (63 MB of 512² x 5 in
 // 1.16 ms against 1.21 by the kernel) and leave the SMs free.
+#include "host_range.h"
 #include "ibpm_internal.cuh"
+
+#include <cuda.h>
 
 namespace ibpm {
 
@@ -33,6 +36,29 @@ __global__ void __launch_bounds__(256) readback_kernel(const double* __restrict_
 }
 
 }  // namespace
+
+// The page-locked range of an address, by the driver's query (the runtime's does
+// not tell the range), all attributes in one call.
+static HostRange host_range(const void* p) {
+    using Query = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+    static const Query query = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        const cudaError_t e = cudaGetDriverEntryPoint("cuPointerGetAttributes", &fn, cudaEnableDefault, &found);
+        return e == cudaSuccess && found == cudaDriverEntryPointSuccess ? reinterpret_cast<Query>(fn) : nullptr;
+    }();
+    unsigned type = 0, managed = 0;
+    CUdeviceptr start = 0, dev = 0;
+    size_t size = 0;
+    CUpointer_attribute want[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                  CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                  CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void* got[] = {&type, &managed, &dev, &start, &size};
+    if (!query || query(5, want, got, reinterpret_cast<CUdeviceptr>(p)) != CUDA_SUCCESS) return {};
+    return {type == CU_MEMORYTYPE_HOST && !managed, static_cast<uintptr_t>(start), size, reinterpret_cast<void*>(dev)};
+}
+
+double* locked_host(const double* host, long long n) { return locked_whole(host, n, host_range); }
 
 cudaError_t launch_pack(const PackArgs& a, int npieces, bool to_device, cudaStream_t st) {
     long long most = 0;

@@ -508,6 +508,8 @@ struct PackPiece {
 };
 struct PackArgs { PackPiece piece[6]; };
 constexpr size_t kPackBytes = (size_t)4 << 20;
+// The device address of n host values that lie in one page-locked range, else null.
+double* locked_host(const double* host, long long n);
 cudaError_t launch_pack(const PackArgs& a, int npieces, bool to_device, cudaStream_t st);
 cudaError_t launch_readback(const double* hist, double* out, int n, const int* status, int* status_out,
                             cudaStream_t st);
