@@ -403,12 +403,13 @@ __global__ void kinematics_kernel(BodyDev b, Geom g, const double* __restrict__ 
     xb[b.nb + p] = yp;
     ub[p] = __dadd_rn(r[4], __dadd_rn(__dmul_rn(__dmul_rn(thd, -s), X), __dmul_rn(__dmul_rn(thd, -c), Y)));
     ub[b.nb + p] = __dadd_rn(r[5], __dadd_rn(__dmul_rn(__dmul_rn(thd, c), X), __dmul_rn(__dmul_rn(thd, -s), Y)));
-    int bx = (int)floor((xp + offx) / h), by = (int)floor((yp + offy) / h);
-    if (!(bx - 6 >= 1 && bx + 6 <= g.nx && by - 6 >= 1 && by + 6 <= g.ny)) {
+    double fx = floor((xp + offx) / h), fy = floor((yp + offy) / h);
+    if (!window_inside(g, fx, fy)) {
         atomicOr(status, 4);
-        bx = min(max(bx, 7), g.nx - 6);
-        by = min(max(by, 7), g.ny - 6);
+        fx = fmin(fmax(fx, 7.0), g.nx - 6.0);            // fmax of no number is 7
+        fy = fmin(fmax(fy, 7.0), g.ny - 6.0);
     }
+    const int bx = (int)fx, by = (int)fy;
     bidx[p] = bx;
     bidx[b.nb + p] = by;
     atomicMin(&bbox[0], bx);

@@ -873,13 +873,12 @@ static int build_coupling(ibpm_handle* h, const ibpm_problem_desc* d) {
     std::vector<int> bidx(2 * nb);
     for (int k = 0; k < nb; ++k) {
         // body_idx = floor((xb + off)/h) (interface-coupling.jl:86-87)
-        bidx[k] = (int)std::floor((d->xb[k] + d->offx) / d->h);
-        bidx[nb + k] = (int)std::floor((d->xb[nb + k] + d->offy) / d->h);
-        const int bx = bidx[k], by = bidx[nb + k];
-        // written so that a point that is no number (INT_MIN) is refused too
-        if (bx < 7 || bx > g.nx - 6 || by < 7 || by > g.ny - 6)
+        const double fx = std::floor((d->xb[k] + d->offx) / d->h), fy = std::floor((d->xb[nb + k] + d->offy) / d->h);
+        if (!window_inside(g, fx, fy))
             return fail(h, IBPM_ERR_INVALID, "body point " + std::to_string(k) +
                                                  ": the 13x13 regularisation stencil leaves the finest grid");
+        bidx[k] = (int)fx;
+        bidx[nb + k] = (int)fy;
     }
     // E reads q = C ψ at fluxes (bidx ± 6): ψ of slab rows by − 8 … by + 5, and
     // the edge values where a window meets the first or last flux of a row or column

@@ -46,6 +46,13 @@ inline Geom make_geom(int nx, int ny, int mg) {
     return g;
 }
 
+// Whether the 13×13 window around body_idx (bx, by) lies inside the finest grid,
+// for the floored coordinates as they are: a value beyond the integers, infinite
+// or no number is outside (as an int it saturates, and bx + 6 would wrap).
+__host__ __device__ inline bool window_inside(const Geom& g, double bx, double by) {
+    return bx >= 7.0 && bx <= g.nx - 6.0 && by >= 7.0 && by <= g.ny - 6.0;
+}
+
 // Maps blockIdx.y (or any flat slab counter) to (batch, level) and offsets.
 struct SlabMap {
     int nlev;            // levels per batch member handled by the launch
