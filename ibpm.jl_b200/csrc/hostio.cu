@@ -2,10 +2,12 @@
 // of the step, by kernels that read and write page-locked host memory directly.
 //
 // A copy engine transfer costs several µs to set up, and a state has up to six
-// pieces; on small grids that is longer than the transfer.  One launch over all
-// pieces: reading 64² x 3 levels (0.6 MB) 68 -> 29 µs, 200² x 3 (4 MB) 230 ->
-// 134 µs.  Above kPackBytes the copy engines are as fast (63 MB of 512² x 5 in
-// 1.16 ms against 1.21 by the kernel) and leave the SMs free.
+// pieces, four of them pitched, which the copy engines write to the device row by
+// row; one launch takes all pieces at the link's rate.  A whole state without q0,
+// page-locked, copies -> kernel: 64² x 3 levels (0.58 MB) read 40.5 -> 28.5 µs,
+// written 131 -> 27; 128² x 5 (3.9 MB) 99 -> 92 and 341 -> 92 µs.  kPackBytes is
+// set by the reads: at 200² x 3 (5.7 MB) they take 131 by copies and 126 by the
+// kernel, at 256² x 5 (15.7 MB) 308 and 314, and copies leave the SMs free.
 #include "host_range.h"
 #include "ibpm_internal.cuh"
 
