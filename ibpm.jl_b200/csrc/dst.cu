@@ -2,10 +2,7 @@
 // (kernels: dst_kernels.cuh, one instantiation unit per length: dst_n<N>.cu).
 #include "dst_kernels.cuh"
 
-#include <math.h>
-
 namespace ibpm {
-
 
 // Every supported transform length N = nx or ny.
 #define IBPM_DST_LENGTHS(X) X(32) X(64) X(128) X(192) X(200) X(256) X(384) X(400) X(512) X(768) X(1024) X(2048)
@@ -47,14 +44,14 @@ static StageDesc stage_desc(int N, int PL) {
     return d;
 }
 
-// Table block of dst_table_doubles(N) = 6N doubles:
-//   FP64: cos(π(t+1)/N) at [0, N), sin(πt/N) at [N, 2N), stage twiddles
-//         exp(+2πi k r/(Ns R)) (complex) from 2N on (≤ N of them);
-//   FP32 (from double 4N on, as floats): 4 sin²(π(t+1)/(2N)) at [0, N),
-//         sin(πt/N) at [N, 2N), the twiddles (complex) from 2N on;
+// Table block of dst_table_doubles(N) = 4.5 N doubles:
+//   FP64: sin(πt/N) at [0, N), stage twiddles exp(+2πi k r/(Ns R)) (complex)
+//         from N on (≤ N of them);
+//   FP32 (from double 3N on, as floats): sin(πt/N) at [0, N), the twiddles
+//         (complex) from N on;
 // each FP32 entry is the FP64 value rounded once.  The throughput plan's
-// twiddles (when built) follow from double 6N on: FP64 (≤ N complex), then
-// FP32 (≤ N complex).
+// twiddles (when built) follow the block: FP64 (≤ N complex), then FP32 (≤ N
+// complex).
 __global__ void dst_twiddles_kernel(StageDesc d, int ntw, double2* W, float2* W32) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ntw; i += gridDim.x * blockDim.x) {
         int st = 0;
@@ -68,19 +65,10 @@ __global__ void dst_twiddles_kernel(StageDesc d, int ntw, double2* W, float2* W3
     }
 }
 
-__global__ void dst_tables_kernel(int N, double* base) {
-    double* c = base;
-    double* s = base + N;
-    float* a32 = reinterpret_cast<float*>(base + 4 * N);
-    float* s32 = a32 + N;
+__global__ void dst_tables_kernel(int N, double* s, float* s32) {
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < N; t += gridDim.x * blockDim.x) {
         s[t] = sinpi((double)t / (double)N);
         s32[t] = (float)s[t];
-        // evaluated as the reference forms the Laplacian eigenvalues:
-        // cos.(π*(1:(n-1))/n) (laplacian.jl:17)
-        c[t] = (t < N - 1) ? cos(M_PI * (double)(t + 1) / (double)N) : 0.0;
-        const double h = sinpi((double)(t + 1) / (2.0 * (double)N));
-        a32[t] = (t < N - 1) ? (float)(4.0 * h * h) : 0.0f;
     }
 }
 
@@ -92,22 +80,20 @@ static cudaError_t twiddles_build(int N, int PL, double2* W, float2* W32, cudaSt
 }
 
 cudaError_t dst_tables_build(int N, double* base, cudaStream_t st) {
-    dst_tables_kernel<<<(N + 255) / 256, 256, 0, st>>>(N, base);
+    const DstPlan p = dst_plan_at(base, N);
+    dst_tables_kernel<<<(N + 255) / 256, 256, 0, st>>>(N, p.s, p.s32);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    return twiddles_build(N, 0, reinterpret_cast<double2*>(base + 2 * N),
-                          reinterpret_cast<float2*>(reinterpret_cast<float*>(base + 4 * N) + 2 * N), st);
+    return twiddles_build(N, 0, p.W, p.W32, st);
 }
 
 DstPlan dst_plan_at(double* base, int N) {
     DstPlan p;
     p.N = N;
-    p.c = base;
-    p.s = base + N;
-    p.W = reinterpret_cast<double2*>(base + 2 * N);
-    p.a32 = reinterpret_cast<float*>(base + 4 * N);
-    p.s32 = p.a32 + N;
-    p.W32 = reinterpret_cast<float2*>(p.a32 + 2 * N);
+    p.s = base;
+    p.W = reinterpret_cast<double2*>(base + N);
+    p.s32 = reinterpret_cast<float*>(base + 3 * N);
+    p.W32 = reinterpret_cast<float2*>(p.s32 + N);
     p.Wt = nullptr;
     p.Wt32 = nullptr;
     p.plan1 = p.planN = DST_PLAN_LATENCY;
@@ -117,14 +103,14 @@ DstPlan dst_plan_at(double* base, int N) {
 
 int dst_plan_create(DstPlan* p, int N, cudaStream_t st) {
     p->N = N;
-    p->W = nullptr; p->s = nullptr; p->c = nullptr;
+    p->W = nullptr; p->s = nullptr;
     if (!dst_supported(N)) return -1;
     double* base = nullptr;
     if (cudaMalloc(&base, sizeof(double) * dst_table_doubles_all(N)) != cudaSuccess) return -2;
     *p = dst_plan_at(base, N);
     if (dst_tables_build(N, base, st) != cudaSuccess) return -2;
-    p->Wt = reinterpret_cast<double2*>(base + 6 * N);
-    p->Wt32 = reinterpret_cast<float2*>(base + 8 * N);
+    p->Wt = reinterpret_cast<double2*>(base + dst_table_doubles(N));
+    p->Wt32 = reinterpret_cast<float2*>(p->Wt + N);
     if (twiddles_build(N, dstk::ct_plan(N, 1), p->Wt, p->Wt32, st) != cudaSuccess) return -2;
     p->planN = DST_PLAN_AUTO;
     if (dst_init_attributes(N) != cudaSuccess) return -2;
@@ -132,9 +118,9 @@ int dst_plan_create(DstPlan* p, int N, cudaStream_t st) {
 }
 
 void dst_plan_destroy(DstPlan* p) {
-    if (p->c) cudaFree(p->c);  // the block starts at c
-    p->W = nullptr; p->s = nullptr; p->c = nullptr;
-    p->W32 = nullptr; p->s32 = nullptr; p->a32 = nullptr;
+    if (p->s) cudaFree(p->s);  // the block starts at s
+    p->W = nullptr; p->s = nullptr;
+    p->W32 = nullptr; p->s32 = nullptr;
     p->Wt = nullptr; p->Wt32 = nullptr;
 }
 

@@ -422,21 +422,19 @@ __device__ __forceinline__ void dst_pair(cplx_t<T>* buf, const cplx_t<T>* W, con
     dst_post<N, TP, G, T>(buf, tid, gid, buf + ct_pad(N), emit);
 }
 
-// Tables of one precision: stage twiddles, sin(π m/N) and the spectral table
-// used by the divide (FP64: cos(π(k+1)/N); FP32: 4 sin²(π(k+1)/(2N))).
+// Tables of one precision: stage twiddles and sin(π m/N).
 template <class T> struct Tabs {
     const cplx_t<T>* W;
     const T* s;
-    const T* c;
 };
 // The stage twiddles are those of plan PL (W / W32: latency plan, Wt / Wt32:
 // throughput plan).
 template <class T> __host__ __device__ Tabs<T> tabs_of(const DstPlan& p, int PL = 0);
 template <> __host__ __device__ inline Tabs<double> tabs_of<double>(const DstPlan& p, int PL) {
-    return {PL ? p.Wt : p.W, p.s, p.c};
+    return {PL ? p.Wt : p.W, p.s};
 }
 template <> __host__ __device__ inline Tabs<float> tabs_of<float>(const DstPlan& p, int PL) {
-    return {PL ? p.Wt32 : p.W32, p.s32, p.a32};
+    return {PL ? p.Wt32 : p.W32, p.s32};
 }
 
 // Copy the transform tables into shared memory: stage twiddles (complex),

@@ -162,18 +162,6 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_al
 
 bool pdl_enabled();
 
-// 1/d by Newton–Raphson: a single-precision seed (relative error ≤ 2^-23),
-// refined twice with r ← r + r(1 − d r), which squares the error each time
-// (2^-46, then below the double rounding).  Within 1-2 ulp of 1/d, with no
-// branches; used where a full IEEE division per element would dominate.
-__device__ __forceinline__ double nr_rcp(double d) {
-    double r = (double)__frcp_rn((float)d);
-    double e = fma(-d, r, 1.0);
-    r = fma(r, e, r);
-    e = fma(-d, r, 1.0);
-    return fma(r, e, r);
-}
-
 template <typename... KArgs, typename... Args>
 cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                      Args... args) {
@@ -196,12 +184,10 @@ cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t sme
 struct DstPlan {
     int N;               // transform length nx = n1 + 1
     double2* W;          // device: per-stage FFT twiddles (stage-contiguous, ≤ N entries)
-    double* s;           // device: sin(π m/N), m < N
-    double* c;           // device: cos(π (k+1)/N), k < N-1 (Laplacian eigenvalues)
+    double* s;           // device: sin(π m/N), m < N (the table block starts here)
     // the same tables rounded to FP32, for the FP32 transforms
     float2* W32;
     float* s32;
-    float* a32;          // 2 (1 − cos(π (k+1)/N)) = 4 sin²(π (k+1)/(2N)), free of cancellation
     // stage twiddles of the throughput plan (radix 8), FP64 and FP32; null
     // when the block holds only the latency plan's tables
     double2* Wt;
@@ -218,10 +204,10 @@ struct DstPlan {
 // unit solves), else the single-slab plan (the levels of one step).
 enum DstPlanKind { DST_PLAN_LATENCY = 0, DST_PLAN_THROUGHPUT = 1, DST_PLAN_AUTO = 2 };
 constexpr int kAutoWideSlabs = 4;
-// Doubles in the table block of one length (FP64 tables, then FP32 tables),
-// and with the throughput plan's twiddles after them.
-inline long long dst_table_doubles(int N) { return 6LL * N; }
-inline long long dst_table_doubles_all(int N) { return 9LL * N; }
+// Doubles in the table block of one length (FP64 tables, then FP32 tables; every
+// length is a multiple of 8), and with the throughput plan's twiddles after them.
+constexpr long long dst_table_doubles(int N) { return 9LL * N / 2; }
+constexpr long long dst_table_doubles_all(int N) { return dst_table_doubles(N) + 3LL * N; }
 
 bool dst_supported(int N);
 int dst_plan_create(DstPlan* p, int N, cudaStream_t st);  // 0 on success

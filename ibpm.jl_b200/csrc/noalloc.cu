@@ -21,11 +21,11 @@ namespace {
 
 constexpr int kMaxN = 512;                                         // nx, ny <= 512
 constexpr size_t kSlabDoubles = (size_t)(kMaxN - 1) * kMaxN;       // (ny-1) rows of pitch nx
-// The supported lengths, each with a fixed block of 6N doubles (FP64 and
-// FP32 tables of one length) at a fixed offset: 6 * 2168 doubles in all.
+// The supported lengths, each with a fixed block of 4.5 N doubles (FP64 and
+// FP32 tables of one length) at a fixed offset: 4.5 * 2168 doubles in all.
 constexpr int kLengths[] = {32, 64, 128, 192, 200, 256, 384, 400, 512};
 constexpr int kNumLengths = sizeof(kLengths) / sizeof(kLengths[0]);
-constexpr size_t table_offset(int k) { return k == 0 ? 0 : table_offset(k - 1) + 6 * (size_t)kLengths[k - 1]; }
+constexpr size_t table_offset(int k) { return k == 0 ? 0 : table_offset(k - 1) + (size_t)dst_table_doubles(kLengths[k - 1]); }
 constexpr size_t kTableDoubles = table_offset(kNumLengths);
 
 __device__ __align__(256) double g_noalloc_slab[kSlabDoubles];
