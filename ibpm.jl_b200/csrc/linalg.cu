@@ -335,7 +335,12 @@ struct GjWork {
     }
 };
 
-// The panel kernel of the fewest rows per thread that holds n rows.
+// The panel kernel of the fewest rows per thread that holds n rows.  Each count is
+// a kernel of its own, so there are three per width: 52 fits the registers (204 to
+// 216 of 255), 80 spills 7 to 12 doubles a thread, 88 some 50, for which a width
+// reaches a tenth further before the next one halves it.  52 and 80 hold the 102
+// components of the pitching plate and the 314 of the 200² cylinder closely; other
+// sizes pay for the rows they leave empty, since a column passes over all K.
 template <int WC>
 cudaError_t gj_panel_w(const double* A, int lda, int n, int c0, int w, double* M, int* piv, unsigned char* used,
                        int* info, int col_base, cudaStream_t st) {
